@@ -1,5 +1,5 @@
 // On-device compact packer: linear splat attributes -> the packed storage
-// buffers the pass consumes (GaussianData.ts:10-33), one thread per splat.
+// buffers the pass consumes (GaussianData.ts:10-33).
 // Restates, on the GPU, the reference's CPU packer for the compact layout:
 //   rust/gaussian-backend/src/engine.rs:1801-1891 encode_attributes (compact):
 //     means          (x, y, z, objectId)
@@ -59,30 +59,37 @@ __device__ uint32_t encode_oct101012(float qx, float qy, float qz, float qw) {
 // the exponent stays e instead of e + 1. Decided exactly: the f32 neighbour
 // of e towards e + 1 lies ulp(e) above a positive e, and below |e| by
 // ulp(|e|) (half that when |e| is a power of two) for a negative e; log2
-// rounds to e when log2(m) is under half that gap. log2(m) is evaluated in
-// double, far more precisely than the decision needs.
-__device__ int rounded_log2_ceil(float mx) {
-  if (isnan(mx)) return 0;       // Rust's saturating cast of NaN
-  if (isinf(mx)) return 127;     // clamped below
-  int ex = 0;
-  const float f = frexpf(mx, &ex);  // mx = f 2^ex, f in [0.5, 1)
-  if (f == 0.5f) return ex - 1;      // a power of two
-  const int e = ex - 1;              // floor(log2 mx); mantissa m = 2 f in (1, 2)
-  if (e == 0) return 1;              // log2 m itself is representable: above 0
+// rounds to e when log2(m) is under half that gap, h = 2^(g - 1). With the
+// mantissa m = 1 + j 2^-23 that is j < 2^23 (2^h - 1) = 2^(g + 22) ln 2 plus
+// a term below 2e-4 (h <= 2^-17), and no 2^(g + 22) ln 2 with g in [-24, -16]
+// lies that close below an integer, so j is compared with the product in
+// FP32 (this was a double log1p per SH word, 16 per splat: the whole kernel
+// ran at the FP64 rate). mx > 0 and not subnormal results below -126 are
+// clamped by the caller.
+__device__ __forceinline__ int rounded_log2_ceil(float mx) {
+  const uint32_t b = __float_as_uint(mx);
+  const int field = (int)(b >> 23);
+  const uint32_t j = b & 0x7fffffu;
+  if (field == 255) return j ? 0 : 127;  // NaN: Rust's saturating cast; infinity is clamped to 127
+  if (field == 0) return -126;           // subnormal: at most -126 before the clamp
+  const int e = field - 127;
+  if (j == 0u) return e;                 // a power of two
+  if (e == 0) return 1;                  // log2 m itself is representable: above 0
   const int a = e > 0 ? e : -e;
-  int gap_exp = (31 - __clz(a)) - 23;
-  if (e < 0 && (a & (a - 1)) == 0) gap_exp -= 1;
-  const double log2_m = log1p((double)(2.0f * f) - 1.0) * 1.4426950408889634074;
-  return log2_m < ldexp(1.0, gap_exp - 1) ? e : e + 1;
+  const int g = (31 - __clz(a)) - 23 - (e < 0 && (a & (a - 1)) == 0 ? 1 : 0);
+  const float limit = __uint_as_float(0x3f317218u + ((uint32_t)(g + 22) << 23));  // 2^(g + 22) ln 2
+  return (float)j < limit ? e : e + 1;
 }
 
 // engine.rs:1940-1949 pack_sh.
-__device__ uint32_t pack_sh(float r, float g, float b) {
+__device__ __forceinline__ uint32_t pack_sh(float r, float g, float b) {
   const float mx = fmaxf(fmaxf(fabsf(r), fabsf(g)), fabsf(b));
   if (mx == 0.0f) return 0u;
   int e = rounded_log2_ceil(mx);
   e = e < -126 ? -126 : (e > 127 ? 127 : e);
-  const float mult = 127.0f / ldexpf(1.0f, e);
+  // 127 / 2^e: exact, 127 = 1.984375 2^6 with the exponent moved by -e, or
+  // infinity past the largest float.
+  const float mult = __uint_as_float(e < -121 ? 0x7f800000u : ((uint32_t)(133 - e) << 23) | 0x7e0000u);
   const float c[3] = {r, g, b};
   uint32_t w = (uint32_t)(e + 127) << 24;
 #pragma unroll
@@ -93,26 +100,48 @@ __device__ uint32_t pack_sh(float r, float g, float b) {
   return w;
 }
 
-__global__ void k_pack(gs3d_splat_source src, uint32_t first, float4* __restrict__ means,
-                       uint2* __restrict__ shape, uint32_t* __restrict__ rot, uint32_t* __restrict__ sh, uint32_t C) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= src.count) return;
-  const size_t slot = (size_t)first + i;
-  const float cx = src.centers[3 * (size_t)i], cy = src.centers[3 * (size_t)i + 1], cz = src.centers[3 * (size_t)i + 2];
-  means[slot] = make_float4(cx, cy, cz, (float)src.object_id);
-  const float sx = src.scales[3 * (size_t)i], sy = src.scales[3 * (size_t)i + 1], sz = src.scales[3 * (size_t)i + 2];
-  shape[slot] = make_uint2(f16_bits(logf(sx)) | (f16_bits(logf(sy)) << 16),
-                           f16_bits(logf(sz)) | (f16_bits(src.opacity[i]) << 16));
-  // glam Quat::normalize: multiply by the reciprocal of the length.
-  const float* q = src.quaternions + 4 * (size_t)i;
-  const float inv = 1.0f / sqrtf(((q[0] * q[0] + q[1] * q[1]) + q[2] * q[2]) + q[3] * q[3]);
-  rot[slot] = encode_oct101012(q[0] * inv, q[1] * inv, q[2] * inv, q[3] * inv);
-  uint32_t* out = sh + slot * C;
-  const float* rgb = src.rgb + 3 * (size_t)i;
-  out[0] = pack_sh((rgb[0] - 0.5f) / kShC0, (rgb[1] - 0.5f) / kShC0, (rgb[2] - 0.5f) / kShC0);
-  for (uint32_t k = 1; k < C; ++k) {
-    const float* c = src.sh_rest + (size_t)i * (C - 1) * 3 + (size_t)(k - 1) * 3;
-    out[k] = pack_sh(c[0], c[1], c[2]);
+constexpr uint32_t kPackBlock = 256;  // splats, and threads, of a block
+
+// HBM-bound: 4 (14 + 3 (C - 1)) bytes read and 28 + 4 C written per splat. A
+// block takes 256 consecutive splats: one thread per splat for the geometry,
+// then its 256 C SH words spread over the threads, so that the coefficient
+// reads (12 consecutive bytes per thread) and the word stores of a warp are
+// consecutive; with a thread per splat they lay C words apart.
+// 1M splats at degree 3: 1810 us with a thread per splat and the double
+// log1p; 92 us (3.6 TB/s) so.
+template <uint32_t C>
+__global__ void __launch_bounds__(kPackBlock) k_pack(gs3d_splat_source src, uint32_t first,
+                                                     float4* __restrict__ means, uint2* __restrict__ shape,
+                                                     uint32_t* __restrict__ rot, uint32_t* __restrict__ sh) {
+  const uint32_t i0 = blockIdx.x * kPackBlock;
+  const uint32_t count = min(kPackBlock, src.count - i0);
+  if (threadIdx.x < count) {
+    const uint32_t i = i0 + threadIdx.x;
+    const size_t slot = (size_t)first + i;
+    const float cx = src.centers[3 * (size_t)i], cy = src.centers[3 * (size_t)i + 1], cz = src.centers[3 * (size_t)i + 2];
+    means[slot] = make_float4(cx, cy, cz, (float)src.object_id);
+    const float sx = src.scales[3 * (size_t)i], sy = src.scales[3 * (size_t)i + 1], sz = src.scales[3 * (size_t)i + 2];
+    shape[slot] = make_uint2(f16_bits(logf(sx)) | (f16_bits(logf(sy)) << 16),
+                             f16_bits(logf(sz)) | (f16_bits(src.opacity[i]) << 16));
+    // glam Quat::normalize: multiply by the reciprocal of the length.
+    const float* q = src.quaternions + 4 * (size_t)i;
+    const float inv = 1.0f / sqrtf(((q[0] * q[0] + q[1] * q[1]) + q[2] * q[2]) + q[3] * q[3]);
+    rot[slot] = encode_oct101012(q[0] * inv, q[1] * inv, q[2] * inv, q[3] * inv);
+  }
+  uint32_t* out = sh + ((size_t)first + i0) * C;
+  const float* rgb = src.rgb + 3 * (size_t)i0;
+  const float* rest = src.sh_rest + (size_t)i0 * (C - 1u) * 3u;
+#pragma unroll 4
+  for (uint32_t w = threadIdx.x; w < count * C; w += kPackBlock) {
+    const uint32_t i = w / C, k = w - i * C;  // word k of the block's splat i
+    float r, g, b;
+    if (k == 0u) {
+      r = (rgb[3u * i] - 0.5f) / kShC0; g = (rgb[3u * i + 1u] - 0.5f) / kShC0; b = (rgb[3u * i + 2u] - 0.5f) / kShC0;
+    } else {
+      const float* c = rest + (w - i - 1u) * 3u;  // (i (C - 1) + k - 1) coefficients precede it
+      r = c[0]; g = c[1]; b = c[2];
+    }
+    out[w] = pack_sh(r, g, b);
   }
 }
 
@@ -129,10 +158,15 @@ extern "C" gs3d_status gs3d_pack_splats(const gs3d_splat_source* src, uint32_t f
       (src->sh_degree > 0 && !src->sh_rest))
     return GS3D_ERROR_INVALID_ARGUMENT;
   if (((uintptr_t)means & 15u) || ((uintptr_t)scales_opacity & 7u)) return GS3D_ERROR_INVALID_ARGUMENT;
-  const uint32_t C = (src->sh_degree + 1) * (src->sh_degree + 1);
-  const uint32_t grid = (src->count + 255u) / 256u;
-  k_pack<<<grid, 256, 0, (cudaStream_t)stream>>>(*src, first_slot, reinterpret_cast<float4*>(means),
-                                                 reinterpret_cast<uint2*>(scales_opacity), rotations,
-                                                 sh_coefficients, C);
+  const uint32_t grid = (src->count - 1u) / kPackBlock + 1u;
+  cudaStream_t st = (cudaStream_t)stream;
+  float4* m = reinterpret_cast<float4*>(means);
+  uint2* s = reinterpret_cast<uint2*>(scales_opacity);
+  switch (src->sh_degree) {
+    case 0: k_pack<1><<<grid, kPackBlock, 0, st>>>(*src, first_slot, m, s, rotations, sh_coefficients); break;
+    case 1: k_pack<4><<<grid, kPackBlock, 0, st>>>(*src, first_slot, m, s, rotations, sh_coefficients); break;
+    case 2: k_pack<9><<<grid, kPackBlock, 0, st>>>(*src, first_slot, m, s, rotations, sh_coefficients); break;
+    default: k_pack<16><<<grid, kPackBlock, 0, st>>>(*src, first_slot, m, s, rotations, sh_coefficients); break;
+  }
   return cudaGetLastError() == cudaSuccess ? GS3D_OK : GS3D_ERROR_CUDA;
 }
