@@ -69,11 +69,88 @@ __device__ __forceinline__ uint32_t bit_range(uint32_t s, uint32_t e) {
 // no per-tile owner lookup, the owner's parameters broadcast to every lane.
 constexpr uint32_t kWideBox = 64;
 
+// The tiles a splat may reach, walked in row-major order: bw columns and bh
+// rows. Along a periodic axis the reference takes every tile of the axis and
+// tests each (projectionHelpers.ts:223-236); the box keeps those that an
+// image of the splat's extent can touch, which is one interval or, across the
+// seam, a first part [0, wrap) and a last part from x0 + wrap (y0 + wrap) on.
+struct TileBox {
+  int x0, y0;
+  uint32_t bw, bh;
+  uint32_t wrap;  // periodic axis: box columns (rows) of the first part
+
+};
+
+// The tile test of box column bx and row by. PERIODIC: o.axis is not 0 (the
+// kernels are compiled for both, so that plain boxes carry no axis tests and
+// no wrap: sharing the code cost the projection 1%).
+template <bool PERIODIC>
+__device__ __forceinline__ int box_column(uint32_t bx, uint32_t x0, uint32_t wrap, uint32_t axis) {
+  return (int)(PERIODIC && axis == 1u && bx < wrap ? bx : x0 + bx);
+}
+template <bool PERIODIC>
+__device__ __forceinline__ int box_row(uint32_t by, uint32_t y0, uint32_t wrap, uint32_t axis) {
+  return (int)(PERIODIC && axis == 2u && by < wrap ? by : y0 + by);
+}
+template <bool PERIODIC>
+__device__ __forceinline__ bool tile_hit(float cx, float cy, float k0, float k1, float k2, float thr, float rx,
+                                         float ry, int tx, int ty, float vw, float vh, uint32_t axis, float ts) {
+  return PERIODIC ? boundary_tile_hit(cx, cy, k0, k1, k2, thr, rx, ry, tx, ty, vw, vh, axis, ts)
+                  : tile_rect_test(cx, cy, k0, k1, k2, thr, tx, ty, ts);
+}
+
+// The tiles of a periodic axis that pass boundary_tile_hit's image range
+// (tileContribution.ts:84-114) for some image, or more: an image centre
+// canon + i period reaches tile t when it lies in [t ts - r, (t + 1) ts + r].
+// The slack of 2 px and a millionth of the period covers the rounding of that
+// range. Every image but i = -1, 0, 1 is out of reach, and at most one of
+// i = -1 and i = 1 in it, when the extent stays well below half the period;
+// otherwise (or with a centre so far out that canon is not in the period)
+// the whole axis is kept. Walking 128 columns for the 2-3 that can hit took
+// 367 us in the projection and 391 us in the emission of 400k splats at
+// 2048x1024 (of 1384 us for the frame; 391 us with this and the rasterizers'
+// fixed image per patch).
+__device__ __forceinline__ void periodic_tiles(float cen, float r, float period, int tiles, float ts, float inv,
+                                               int* start, uint32_t* count, uint32_t* wrap) {
+  *start = 0; *count = (uint32_t)tiles; *wrap = 0u;
+  const float canon = cen - floorf(cen / period) * period;
+  const float reach = r + 2.0f + 1e-6f * period;
+  if (!(canon >= 0.0f && canon <= period && 2.0f * (reach + ts) < period)) return;
+  const int last = tiles - 1;
+  const int a = max((int)floorf((canon - reach) * inv), 0), b = min((int)floorf((canon + reach) * inv), last);
+  const float before = canon - period + reach, after = canon + period - reach;
+  if (before >= 0.0f) {  // image -1 reaches the first tiles, image 0 the last one
+    const int n0 = (int)floorf(before * inv) + 1;
+    *wrap = (uint32_t)n0; *start = a - n0; *count = (uint32_t)(n0 + tiles - a);
+  } else if (after <= (float)tiles * ts) {  // image 1 reaches the last tiles, image 0 the first one
+    const int f = min((int)floorf(after * inv), last), n0 = b + 1;
+    *wrap = (uint32_t)n0; *start = f - n0; *count = (uint32_t)(n0 + tiles - f);
+  } else {
+    *start = a; *count = (uint32_t)(b - a + 1);
+  }
+}
+
+template <bool PERIODIC>
+__device__ __forceinline__ TileBox tile_box(float cx, float cy, float rx, float ry, float vw, float vh, int tiles_x,
+                                            int tiles_y, const PassOptions& o) {
+  const float mtx = (float)(tiles_x - 1), mty = (float)(tiles_y - 1);
+  // Division by the tile side, a power of two: the product with its
+  // reciprocal is the same correctly rounded value.
+  const int tminx = (int)clampf(floorf((cx - rx) * o.tile_inv), 0.0f, mtx);
+  const int tminy = (int)clampf(floorf((cy - ry) * o.tile_inv), 0.0f, mty);
+  const int tmaxx = (int)clampf(floorf((cx + rx) * o.tile_inv), 0.0f, mtx);
+  const int tmaxy = (int)clampf(floorf((cy + ry) * o.tile_inv), 0.0f, mty);
+  TileBox t = {tminx, tminy, (uint32_t)(tmaxx - tminx + 1), (uint32_t)(tmaxy - tminy + 1), 0u};
+  if (PERIODIC && o.axis == 1u) periodic_tiles(cx, rx, vw, tiles_x, o.tile_px, o.tile_inv, &t.x0, &t.bw, &t.wrap);
+  if (PERIODIC && o.axis == 2u) periodic_tiles(cy, ry, vh, tiles_y, o.tile_px, o.tile_inv, &t.y0, &t.bh, &t.wrap);
+  return t;
+}
+
 // Per-warp tables of the projection's cooperative tile count: the splat
 // parameters of the tile test, the box, and the inclusive box-tile counts.
 struct CountShared {
   float f[8][kBlock / 32][32];     // cx, cy, conic a, b, c, threshold, rx, ry
-  uint32_t u[4][kBlock / 32][32];  // tminx, tminy, box width, box index of the centre tile (or ~0)
+  uint32_t u[5][kBlock / 32][32];  // box x0, y0, width, box index of the centre tile (or ~0), wrap
   uint32_t incl[kBlock / 32][32];
   uint32_t cnt[kBlock / 32][32];
 };
@@ -86,6 +163,7 @@ struct CountShared {
 // walked afterwards by the whole warp, one at a time. Must be called by all
 // 32 lanes; a lane with nbox == 0 contributes nothing. Returns the lane's
 // count.
+template <bool PERIODIC>
 __device__ __forceinline__ uint32_t count_tiles_warp(CountShared& sm, uint32_t nbox, float vw, float vh,
                                                      uint32_t axis, float ts) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -115,10 +193,11 @@ __device__ __forceinline__ uint32_t count_tiles_warp(CountShared& sm, uint32_t n
       uint32_t k = j - (owner ? sm.incl[warp][owner - 1] : 0u);
       k += k >= sm.u[3][warp][owner] ? 1u : 0u;
       const uint32_t by = k / bw, bx = k - by * bw;
-      hit = boundary_tile_hit(sm.f[0][warp][owner], sm.f[1][warp][owner], sm.f[2][warp][owner],
+      hit = tile_hit<PERIODIC>(sm.f[0][warp][owner], sm.f[1][warp][owner], sm.f[2][warp][owner],
                               sm.f[3][warp][owner], sm.f[4][warp][owner], sm.f[5][warp][owner],
-                              sm.f[6][warp][owner], sm.f[7][warp][owner], (int)(sm.u[0][warp][owner] + bx),
-                              (int)(sm.u[1][warp][owner] + by), vw, vh, axis, ts);
+                              sm.f[6][warp][owner], sm.f[7][warp][owner],
+                              box_column<PERIODIC>(bx, sm.u[0][warp][owner], sm.u[4][warp][owner], axis),
+                              box_row<PERIODIC>(by, sm.u[1][warp][owner], sm.u[4][warp][owner], axis), vw, vh, axis, ts);
     }
     const uint32_t hits = __ballot_sync(0xffffffffu, hit);
     const uint32_t same = __match_any_sync(0xffffffffu, valid ? owner : 32u + lane);
@@ -144,9 +223,10 @@ __device__ __forceinline__ uint32_t count_tiles_warp(CountShared& sm, uint32_t n
         k += k >= vu[3][warp][w] ? 1u : 0u;
         const uint32_t bw = vu[2][warp][w];
         const uint32_t by = k / bw, bx = k - by * bw;
-        hit = boundary_tile_hit(vf[0][warp][w], vf[1][warp][w], vf[2][warp][w], vf[3][warp][w], vf[4][warp][w],
-                                vf[5][warp][w], vf[6][warp][w], vf[7][warp][w], (int)(vu[0][warp][w] + bx),
-                                (int)(vu[1][warp][w] + by), vw, vh, axis, ts);
+        hit = tile_hit<PERIODIC>(vf[0][warp][w], vf[1][warp][w], vf[2][warp][w], vf[3][warp][w], vf[4][warp][w],
+                                vf[5][warp][w], vf[6][warp][w], vf[7][warp][w],
+                                box_column<PERIODIC>(bx, vu[0][warp][w], vu[4][warp][w], axis),
+                                box_row<PERIODIC>(by, vu[1][warp][w], vu[4][warp][w], axis), vw, vh, axis, ts);
       }
       sum += __popc(__ballot_sync(0xffffffffu, hit));
     }
@@ -158,7 +238,7 @@ __device__ __forceinline__ uint32_t count_tiles_warp(CountShared& sm, uint32_t n
 // GROUPED: some group holds several views (decode once, before the view
 // loop); otherwise every group is one view and the decode stays inside the
 // per-view chain, after the object tests, where it costs fewest registers.
-template <bool FP64, bool GROUPED, bool FAST_SH>
+template <bool FP64, bool GROUPED, bool FAST_SH, bool PERIODIC>
 __global__ void __launch_bounds__(kBlock, 4) k_project(BatchView b, PassOptions o, float4* __restrict__ mean_out,
                                                     float4* __restrict__ conic_out, float4* __restrict__ color_out,
                                                     uint32_t* __restrict__ count_out, uint32_t* __restrict__ key_out,
@@ -277,37 +357,27 @@ __global__ void __launch_bounds__(kBlock, 4) k_project(BatchView b, PassOptions 
         mo4 = make_float4(pr.cx, pr.cy, pr.depth, -1.0f);  // subpixel marker (:572-587)
         break;
       }
-      const int tiles_x = (int)v.tiles_x, tiles_y = (int)v.tiles_y;
-      const float mtx = (float)(tiles_x - 1), mty = (float)(tiles_y - 1);
-      // Division by the tile side, a power of two: the product with its
-      // reciprocal is the same correctly rounded value.
-      const float fx0 = floorf(bminx * o.tile_inv), fy0 = floorf(bminy * o.tile_inv);
-      const float fx1 = floorf(bmaxx * o.tile_inv), fy1 = floorf(bmaxy * o.tile_inv);
-      int tminx = (int)clampf(fx0, 0.0f, mtx);
-      int tminy = (int)clampf(fy0, 0.0f, mty);
-      int tmaxx = (int)clampf(fx1, 0.0f, mtx);
-      int tmaxy = (int)clampf(fy1, 0.0f, mty);
-      if (o.axis == 1u) { tminx = 0; tmaxx = tiles_x - 1; }
-      if (o.axis == 2u) { tminy = 0; tmaxy = tiles_y - 1; }
-      const uint32_t bw = (uint32_t)(tmaxx - tminx + 1);
-      nbox = bw * (uint32_t)(tmaxy - tminy + 1);
+      const TileBox box = tile_box<PERIODIC>(pr.cx, pr.cy, rx, ry, vw, vh, (int)v.tiles_x, (int)v.tiles_y, o);
+      const float mtx = (float)((int)v.tiles_x - 1), mty = (float)((int)v.tiles_y - 1);
+      nbox = box.bw * box.bh;
       // The tile holding the centre, when it is on screen, lies in the box
       // (the floors are monotone and rx, ry >= 1) and passes the reference's
       // tile test by its centre-inside path (tileContribution.ts:16-59): it
       // counts 1 without a test, and the warp walks the box's other tiles.
       const float fcx = floorf(pr.cx * o.tile_inv), fcy = floorf(pr.cy * o.tile_inv);
-      centre = o.axis == 0u && fcx >= 0.0f && fcx <= mtx && fcy >= 0.0f && fcy <= mty;
+      centre = !PERIODIC && fcx >= 0.0f && fcx <= mtx && fcy >= 0.0f && fcy <= mty;
       s_count.u[3][warp][lane] =
-          centre ? ((uint32_t)fcy - (uint32_t)tminy) * bw + ((uint32_t)fcx - (uint32_t)tminx) : 0xffffffffu;
+          centre ? ((uint32_t)fcy - (uint32_t)box.y0) * box.bw + ((uint32_t)fcx - (uint32_t)box.x0) : 0xffffffffu;
       s_count.f[0][warp][lane] = pr.cx; s_count.f[1][warp][lane] = pr.cy;
       s_count.f[2][warp][lane] = pr.conic_x; s_count.f[3][warp][lane] = pr.conic_y;
       s_count.f[4][warp][lane] = pr.conic_z; s_count.f[5][warp][lane] = thr;
       s_count.f[6][warp][lane] = rx; s_count.f[7][warp][lane] = ry;
-      s_count.u[0][warp][lane] = (uint32_t)tminx; s_count.u[1][warp][lane] = (uint32_t)tminy;
-      s_count.u[2][warp][lane] = bw;
+      s_count.u[0][warp][lane] = (uint32_t)box.x0; s_count.u[1][warp][lane] = (uint32_t)box.y0;
+      s_count.u[2][warp][lane] = box.bw;
+      if (PERIODIC) s_count.u[4][warp][lane] = box.wrap;
     } while (false);
     // Tiles passing the tile test (projectionHelpers.ts:223-236), counted by the whole warp.
-    cnt = count_tiles_warp(s_count, centre ? nbox - 1u : nbox, vw, vh, o.axis, o.tile_px) + (centre ? 1u : 0u);
+    cnt = count_tiles_warp<PERIODIC>(s_count, centre ? nbox - 1u : nbox, vw, vh, o.axis, o.tile_px) + (centre ? 1u : 0u);
     if (cnt > 0) {
       uint32_t co[16];
       load_sh(v.sh + (size_t)slot * v.C, v.degree, co);
@@ -358,12 +428,16 @@ template <bool FAST_SH>
 void launch_project_t(const BatchView& b, const PassOptions& o, float4* mean, float4* conic, float4* color,
                       uint32_t* counts, uint32_t* keys, float4* rec, float4* erec, cudaStream_t st) {
   const bool grouped = b.ngroups < b.nviews;
-#define GS_PROJECT(F, G) \
-  k_project<F, G, FAST_SH><<<b.total_blocks, kBlock, 0, st>>>(b, o, mean, conic, color, counts, keys, rec, erec)
+#define GS_PROJECT(F, G)                                                                                          \
+  if (o.axis)                                                                                                     \
+    k_project<F, G, FAST_SH, true>                                                                                \
+        <<<b.total_blocks, kBlock, 0, st>>>(b, o, mean, conic, color, counts, keys, rec, erec);                   \
+  else                                                                                                            \
+    k_project<F, G, FAST_SH, false><<<b.total_blocks, kBlock, 0, st>>>(b, o, mean, conic, color, counts, keys, rec, erec)
   if (o.proj_fp64) {
-    if (grouped) GS_PROJECT(true, true); else GS_PROJECT(true, false);
+    if (grouped) { GS_PROJECT(true, true); } else { GS_PROJECT(true, false); }
   } else {
-    if (grouped) GS_PROJECT(false, true); else GS_PROJECT(false, false);
+    if (grouped) { GS_PROJECT(false, true); } else { GS_PROJECT(false, false); }
   }
 #undef GS_PROJECT
 }
@@ -651,8 +725,8 @@ constexpr int kEmitWarps = kBlock / 32;
 
 struct EmitShared {
   float f[10][kEmitWarps][32];     // cx, cy, conic a, b, c, threshold, rx, ry, view width, height
-  uint32_t u[9][kEmitWarps][32];   // tminx, tminy, box width, tiles_x, tile_base, base, reserved, item,
-                                   // first box tile of the warp's walk
+  uint32_t u[10][kEmitWarps][32];  // box x0, y0, width, tiles_x, tile_base, base, reserved, item,
+                                   // first box tile of the warp's walk, wrap
   uint32_t own[kEmitWarps][32];    // lane owning the k-th segment of the round
   uint32_t filled[kEmitWarps][32]; // records placed so far per rank
 };
@@ -661,6 +735,7 @@ struct EmitShared {
 // tile-test inputs for its warp, walk the union of the warp's boxes 32 box
 // tiles per round, place hits after the owner's earlier hits, pad with
 // sentinels. The lane's rank data were loaded by the caller.
+template <bool PERIODIC>
 __device__ __forceinline__ void emit_group(EmitShared& sm, bool live, uint32_t g, float4 e0, float4 e1,
                                            uint32_t reserved, uint32_t base_off, const BatchView& bv,
                                            const PassOptions& o, uint32_t capacity, uint32_t* __restrict__ tile_keys,
@@ -676,23 +751,16 @@ __device__ __forceinline__ void emit_group(EmitShared& sm, bool live, uint32_t g
     const uint32_t packed = (uint32_t)e1.z;
     const float rx = (float)(packed % 512u), ry = (float)(packed / 512u);
     const float thr = e1.y;  // log(opacity * 255), computed by the projection
-    const int tiles_x = (int)v.tiles_x, tiles_y = (int)v.tiles_y;
-    const float mtx = (float)(tiles_x - 1), mty = (float)(tiles_y - 1);
-    int tminx = (int)clampf(floorf((m.x - rx) * o.tile_inv), 0.0f, mtx);
-    int tminy = (int)clampf(floorf((m.y - ry) * o.tile_inv), 0.0f, mty);
-    int tmaxx = (int)clampf(floorf((m.x + rx) * o.tile_inv), 0.0f, mtx);
-    int tmaxy = (int)clampf(floorf((m.y + ry) * o.tile_inv), 0.0f, mty);
-    if (o.axis == 1u) { tminx = 0; tmaxx = tiles_x - 1; }
-    if (o.axis == 2u) { tminy = 0; tmaxy = tiles_y - 1; }
-    const uint32_t bw = (uint32_t)(tmaxx - tminx + 1);
+    const TileBox box = tile_box<PERIODIC>(m.x, m.y, rx, ry, v.vw, v.vh, (int)v.tiles_x, (int)v.tiles_y, o);
     // A rank with nothing reserved emits nothing; its box takes no rounds.
-    nbox = reserved ? bw * (uint32_t)(tmaxy - tminy + 1) : 0u;
+    nbox = reserved ? box.bw * box.bh : 0u;
     sm.f[0][warp][lane] = m.x; sm.f[1][warp][lane] = m.y;
     sm.f[2][warp][lane] = c.x; sm.f[3][warp][lane] = c.y; sm.f[4][warp][lane] = c.z;
     sm.f[5][warp][lane] = thr; sm.f[6][warp][lane] = rx; sm.f[7][warp][lane] = ry;
     sm.f[8][warp][lane] = v.vw; sm.f[9][warp][lane] = v.vh;
-    sm.u[0][warp][lane] = (uint32_t)tminx; sm.u[1][warp][lane] = (uint32_t)tminy; sm.u[2][warp][lane] = bw;
-    sm.u[3][warp][lane] = (uint32_t)tiles_x; sm.u[4][warp][lane] = v.tile_base;
+    sm.u[0][warp][lane] = (uint32_t)box.x0; sm.u[1][warp][lane] = (uint32_t)box.y0; sm.u[2][warp][lane] = box.bw;
+    sm.u[3][warp][lane] = v.tiles_x; sm.u[4][warp][lane] = v.tile_base;
+    if (PERIODIC) sm.u[9][warp][lane] = box.wrap;
     sm.u[5][warp][lane] = base_off; sm.u[6][warp][lane] = reserved; sm.u[7][warp][lane] = g;
   }
   const uint32_t le = lt | (1u << lane);
@@ -741,9 +809,10 @@ __device__ __forceinline__ void emit_group(EmitShared& sm, bool live, uint32_t g
         const uint32_t bw = sm.u[2][warp][owner];
         const uint32_t kk = j - sm.u[8][warp][owner];
         const uint32_t by = kk / bw, bx = kk - by * bw;
-        const int tx = (int)(sm.u[0][warp][owner] + bx), ty = (int)(sm.u[1][warp][owner] + by);
+        const int tx = box_column<PERIODIC>(bx, sm.u[0][warp][owner], sm.u[9][warp][owner], o.axis);
+        const int ty = box_row<PERIODIC>(by, sm.u[1][warp][owner], sm.u[9][warp][owner], o.axis);
         hit = pass == 0 ||
-              boundary_tile_hit(sm.f[0][warp][owner], sm.f[1][warp][owner], sm.f[2][warp][owner],
+              tile_hit<PERIODIC>(sm.f[0][warp][owner], sm.f[1][warp][owner], sm.f[2][warp][owner],
                                 sm.f[3][warp][owner], sm.f[4][warp][owner], sm.f[5][warp][owner],
                                 sm.f[6][warp][owner], sm.f[7][warp][owner], tx, ty, sm.f[8][warp][owner],
                                 sm.f[9][warp][owner], o.axis, o.tile_px);
@@ -790,8 +859,9 @@ __device__ __forceinline__ void emit_group(EmitShared& sm, bool live, uint32_t g
       if (k < wn) {
         const uint32_t wbw = vu[2][warp][w];
         const uint32_t by = k / wbw, bx = k - by * wbw;
-        const int tx = (int)(vu[0][warp][w] + bx), ty = (int)(vu[1][warp][w] + by);
-        hit = wfull || boundary_tile_hit(vf[0][warp][w], vf[1][warp][w], vf[2][warp][w], vf[3][warp][w],
+        const int tx = box_column<PERIODIC>(bx, vu[0][warp][w], vu[9][warp][w], o.axis);
+        const int ty = box_row<PERIODIC>(by, vu[1][warp][w], vu[9][warp][w], o.axis);
+        hit = wfull || tile_hit<PERIODIC>(vf[0][warp][w], vf[1][warp][w], vf[2][warp][w], vf[3][warp][w],
                                          vf[4][warp][w], vf[5][warp][w], vf[6][warp][w], vf[7][warp][w], tx, ty,
                                          vf[8][warp][w], vf[9][warp][w], o.axis, o.tile_px);
         t = vu[4][warp][w] + (uint32_t)ty * vu[3][warp][w] + (uint32_t)tx;
@@ -828,7 +898,7 @@ __device__ __forceinline__ void emit_group(EmitShared& sm, bool live, uint32_t g
 // launches (many blocks in flight anyway); one keeps small launches wide.
 constexpr uint32_t kEmitTwoGroupsFrom = 1u << 23;  // ranks per launch
 
-template <int G>
+template <int G, bool PERIODIC>
 __global__ void __launch_bounds__(kBlock) k_emit(const uint32_t* __restrict__ ids, const float4* __restrict__ erec,
                                                  const uint32_t* __restrict__ ordered,
                                                  const uint32_t* __restrict__ offsets, BatchView bv, PassOptions o,
@@ -864,7 +934,7 @@ __global__ void __launch_bounds__(kBlock) k_emit(const uint32_t* __restrict__ id
 #pragma unroll
   for (int h = 0; h < G; ++h) {
     const uint32_t r = first + (uint32_t)h * kBlock + tid;
-    emit_group(sm, r < n, g[h], e0[h], e1[h], res[h], off[h], bv, o, capacity, tile_keys, tile_vals);
+    emit_group<PERIODIC>(sm, r < n, g[h], e0[h], e1[h], res[h], off[h], bv, o, capacity, tile_keys, tile_vals);
   }
 }
 
@@ -872,15 +942,16 @@ void launch_emit(const uint32_t* ids, uint32_t n_max, const float4* erec, const 
                  const uint32_t* offsets, const BatchView& b, const PassOptions& o, Control* ctl, uint32_t capacity,
                  uint32_t* tile_keys, uint32_t* tile_vals, cudaStream_t st) {
   if (n_max == 0) return;
-  if (n_max >= kEmitTwoGroupsFrom) {
-    const uint32_t grid = (n_max + 2 * kBlock - 1) / (2 * kBlock);
-    k_emit<2><<<grid, kBlock, 0, st>>>(ids, erec, ordered, offsets, b, o, ctl, capacity, tile_keys,
-                                       tile_vals);
+  const uint32_t per = n_max >= kEmitTwoGroupsFrom ? 2u * kBlock : kBlock;
+  const uint32_t grid = (n_max - 1u) / per + 1u;
+#define GS_EMIT(G, P) \
+  k_emit<G, P><<<grid, kBlock, 0, st>>>(ids, erec, ordered, offsets, b, o, ctl, capacity, tile_keys, tile_vals)
+  if (per == kBlock) {
+    if (o.axis) GS_EMIT(1, true); else GS_EMIT(1, false);
   } else {
-    const uint32_t grid = (n_max + kBlock - 1) / kBlock;
-    k_emit<1><<<grid, kBlock, 0, st>>>(ids, erec, ordered, offsets, b, o, ctl, capacity, tile_keys,
-                                       tile_vals);
+    if (o.axis) GS_EMIT(2, true); else GS_EMIT(2, false);
   }
+#undef GS_EMIT
 }
 
 // ---------------------------------------------------------------------------

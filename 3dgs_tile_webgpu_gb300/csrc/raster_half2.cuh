@@ -103,12 +103,53 @@ __device__ __forceinline__ float2 cholesky_alpha(const uint4& h, __half2 ux, __h
   return __half22float2(h2ex2_approx(__hmin2(u2h2(q), __float2half2_rn(kLog2MaxAlpha))));
 }
 
+// Periodic boundaries: which image of the record the warp's patch sees, for
+// staging. Most splats are far smaller than the period: their one image that
+// the patch can see (single_image) is fixed here, the record is culled against
+// the patch at that image, and its pixels take dx, dy by one multiply-add
+// instead of boundary_delta's two divisions. *image is its index, or NaN
+// for a record whose pixels choose their image one by one (when every record
+// did, and none was culled, the rasterizer took 465 us for 400k splats at
+// 2048x1024; the whole frame takes 391 us so).
+// r0 becomes the record at the canonical centre. (wx, wy): the patch's extent
+// between its first and last pixel centres, from (x0, y0).
+__device__ __forceinline__ bool periodic_reach(float4& r0, const float4& r1, const RasterFrame& f, float x0, float y0,
+                                               float wx, float wy, float* image) {
+  const float A = -r0.z, B = -r0.w, C = -r1.x;
+  const float det4 = 4.0f * A * C - B * B;
+  const float tr = A + C;
+  const float R = fmaf(r1.y + 7.99435329f, 1.01f, 0.01f);
+  *image = __int_as_float(0x7fc00000);
+  if (!(A > 0.0f) || !(C > 0.0f) || !(det4 > 0.0f) || !(tr * tr <= 1e4f * det4)) return true;
+  // Half the support's extent along the axis, widened like patch_mask's.
+  const float h = sqrtf(__fdividef(4.0f * R * (f.axis == 1u ? C : A), det4)) * 1.05f + 0.25f;
+  if (!single_image(h, f)) return true;  // NaN (nothing passes the alpha test): one by one
+  r0.x = canonical_x(r0.x, f);
+  r0.y = canonical_y(r0.y, f);
+  const float k = f.axis == 1u ? nearest_image(r0.x, x0 + 0.5f * wx, f.vw) : nearest_image(r0.y, y0 + 0.5f * wy, f.vh);
+  *image = k;
+  const float cx = f.axis == 1u ? fmaf(k, f.vw, r0.x) : r0.x, cy = f.axis == 2u ? fmaf(k, f.vh, r0.y) : r0.y;
+  return patch_reach(cx, cy, r0.z, r0.w, r1.x, r1.y, x0, y0, wx, wy);
+}
+
+// The pixel's offset from the staged record g (raw: conic and image).
+__device__ __forceinline__ void periodic_delta(float pxc, float pyc, const float4& g, const float4& raw,
+                                               const RasterFrame& f, float* dx, float* dy) {
+  if (raw.w != raw.w) {
+    boundary_delta<true>(pxc, pyc, g.x, g.y, raw.x, raw.y, raw.z, f, dx, dy);
+    return;
+  }
+  const float ddx = pxc - g.x, ddy = pyc - g.y;
+  *dx = f.axis == 1u ? ddx - raw.w * f.vw : ddx;
+  *dy = f.axis == 2u ? ddy - raw.w * f.vh : ddy;
+}
+
 // One warp's staged records (up to 32, compacted in record order).
 struct WarpStage {
   float4 geo[32];  // cx, cy, -a/2 log2 e, -b log2 e (the half2 form: its Cholesky record)
   float4 con[32];  // -c/2 log2 e, log2 opacity, L as half2 bits, depth
   float4 col[32];  // r, g, b (the half2 form: and depth)
-  float4 raw[32];  // conic (a, b, c) for periodic boundaries
+  float4 raw[32];  // conic (a, b, c) and image index for periodic boundaries
   uint8_t idx[32]; // lane (record offset within the group) of each staged record
 };
 
@@ -159,7 +200,7 @@ __device__ __forceinline__ void blend_range_h2(uint32_t begin, uint32_t source_c
     const uint32_t i = b + lane;
     bool reach = false;
     float4 r0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), r1 = r0, col32 = r0;
-    float depth = 0.0f;
+    float depth = 0.0f, image = 0.0f;
     uint32_t cur_id = 0;
     if (!HALF) {
       cur_id = next_id;
@@ -171,8 +212,9 @@ __device__ __forceinline__ void blend_range_h2(uint32_t begin, uint32_t source_c
       r1 = __ldg(rec + 2 * (size_t)g + 1);
       if (!HALF) col32 = __ldg(color + g);
       if (DEPTH && need_depth) depth = __ldg(&mean[g].z);
-      reach = PERIODIC || patch_reach(r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, patch_x0 + 0.5f, patch_y0 + 0.5f,
-                                          7.0f, 7.0f);
+      reach = PERIODIC ? periodic_reach(r0, r1, f, patch_x0 + 0.5f, patch_y0 + 0.5f, 7.0f, 7.0f, &image)
+                       : patch_reach(r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, patch_x0 + 0.5f, patch_y0 + 0.5f, 7.0f,
+                                     7.0f);
     }
     const uint32_t bal = __ballot_sync(0xffffffffu, reach);
     if (reach) {
@@ -195,7 +237,10 @@ __device__ __forceinline__ void blend_range_h2(uint32_t begin, uint32_t source_c
           ws.col[q] = col32;
         }
       }
-      if (PERIODIC) ws.raw[q] = raw_conic(r0, r1);
+      if (PERIODIC) {
+        ws.raw[q] = raw_conic(r0, r1);
+        ws.raw[q].w = image;
+      }
       if (STATS) ws.idx[q] = (uint8_t)lane;
     }
     __syncwarp();
@@ -237,8 +282,8 @@ __device__ __forceinline__ void blend_range_h2(uint32_t begin, uint32_t source_c
       if (PERIODIC) {
         const float4 r = ws.raw[j];
         float dx0, dy0, dx1, dy1;
-        boundary_delta<true>(pxc, pyc0, g.x, g.y, r.x, r.y, r.z, f, &dx0, &dy0);
-        boundary_delta<true>(pxc, pyc1, g.x, g.y, r.x, r.y, r.z, f, &dx1, &dy1);
+        periodic_delta(pxc, pyc0, g, r, f, &dx0, &dy0);
+        periodic_delta(pxc, pyc1, g, r, f, &dx1, &dy1);
         p0 = fmaf(g.z * dx0, dx0, fmaf(g.w * dx0, dy0, fmaf(c.x * dy0, dy0, c.y)));
         p1 = fmaf(g.z * dx1, dx1, fmaf(g.w * dx1, dy1, fmaf(c.x * dy1, dy1, c.y)));
       } else {
@@ -356,7 +401,7 @@ __device__ __forceinline__ void blend_range_hk(uint32_t begin, uint32_t source_c
     const uint32_t i = b + lane;
     bool reach = false;
     float4 r0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), r1 = r0, col32 = r0;
-    float depth = 0.0f;
+    float depth = 0.0f, image = 0.0f;
     uint32_t cur_id = 0;
     if (!HALF) {
       cur_id = next_id;
@@ -368,8 +413,10 @@ __device__ __forceinline__ void blend_range_hk(uint32_t begin, uint32_t source_c
       r1 = __ldg(rec + 2 * (size_t)g + 1);
       if (!HALF) col32 = __ldg(color + g);
       if (DEPTH && need_depth) depth = __ldg(&mean[g].z);
-      reach = PERIODIC || patch_reach(r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, patch_x0 + 0.5f, patch_y0 + 0.5f,
-                                          7.0f, 4.0f * (float)K - 1.0f);
+      reach = PERIODIC ? periodic_reach(r0, r1, f, patch_x0 + 0.5f, patch_y0 + 0.5f, 7.0f,
+                                        4.0f * (float)K - 1.0f, &image)
+                       : patch_reach(r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, patch_x0 + 0.5f, patch_y0 + 0.5f, 7.0f,
+                                     4.0f * (float)K - 1.0f);
     }
     const uint32_t bal = __ballot_sync(0xffffffffu, reach);
     if (reach) {
@@ -392,7 +439,10 @@ __device__ __forceinline__ void blend_range_hk(uint32_t begin, uint32_t source_c
           ws.col[q] = col32;
         }
       }
-      if (PERIODIC) ws.raw[q] = raw_conic(r0, r1);
+      if (PERIODIC) {
+        ws.raw[q] = raw_conic(r0, r1);
+        ws.raw[q].w = image;
+      }
       if (STATS) ws.idx[q] = (uint8_t)lane;
     }
     __syncwarp();
@@ -443,7 +493,7 @@ __device__ __forceinline__ void blend_range_hk(uint32_t begin, uint32_t source_c
 #pragma unroll
         for (int k = 0; k < K; ++k) {
           float dx, dy;
-          boundary_delta<true>(pxc, pyc[k], g.x, g.y, r.x, r.y, r.z, f, &dx, &dy);
+          periodic_delta(pxc, pyc[k], g, r, f, &dx, &dy);
           pv[k] = fmaf(g.z * dx, dx, fmaf(g.w * dx, dy, fmaf(c.x * dy, dy, c.y)));
         }
       } else {

@@ -95,6 +95,29 @@ __device__ __forceinline__ void boundary_delta(float pxc, float pyc, float cx, f
   *dy = ddy;
 }
 
+// The centre's image inside the period of a periodic axis (the expressions of
+// boundary_delta, so the same bits).
+__device__ __forceinline__ float canonical_x(float cx, const RasterFrame& f) {
+  return f.axis == 1u ? cx - floorf(cx / f.vw) * f.vw : cx;
+}
+__device__ __forceinline__ float canonical_y(float cy, const RasterFrame& f) {
+  return f.axis == 2u ? cy - floorf(cy / f.vh) * f.vh : cy;
+}
+
+// Whether a splat whose support reaches h along the periodic axis shows at
+// most one image to the pixels of any patch (at most 16 pixels long). The
+// pixels p of a patch that pass the alpha test have |p - centre - k period|
+// <= h for the image k that boundary_delta picks; with 2 h + 18 below the
+// period, every such k is the image nearest to the patch's middle. Any other
+// pixel of the patch fails the test at every image, boundary_delta's
+// minimising one included.
+__device__ __forceinline__ bool single_image(float h, const RasterFrame& f) {
+  return 2.0f * h + 18.0f < (f.axis == 1u ? f.vw : f.vh);
+}
+__device__ __forceinline__ float nearest_image(float canon, float middle, float period) {
+  return rintf((middle - canon) / period);
+}
+
 struct PixelAcc {
   float r, g, b, t, d;
 };
@@ -121,13 +144,15 @@ constexpr float kLog2MaxAlpha = -0.01449957f;  // log2(0.99)
 // 32 w. Conservative: the support's
 // bounding box is widened by 5 % + 0.25 px, far beyond the rounding of the
 // per-pixel evaluation for conics whose condition number is below 4e4 (the
-// 0.3 px^2 filter bounds it near 3.3e4); worse-conditioned splats, periodic
-// boundaries and non-finite values keep every bit set.
+// 0.3 px^2 filter bounds it near 3.3e4); worse-conditioned splats and
+// non-finite values keep every bit set. With a periodic boundary the box is
+// tested at the splat's image nearest to each patch, the only one a pixel of
+// the patch can see while the extent is below half the period
+// (nearest_image); larger splats keep every bit set.
 template <int NW>
 __device__ __forceinline__ uint32_t patch_mask(float cx, float cy, float ca, float cb, float cc, float thr,
-                                               float tile_x0, float tile_y0, uint32_t axis) {
+                                               float tile_x0, float tile_y0, const RasterFrame& f) {
   constexpr uint32_t kAll = NW >= 32 ? 0xffffffffu : (1u << NW) - 1u;
-  if (axis != 0u) return kAll;
   const float det = ca * cc - cb * cb;
   const float tr = ca + cc;
   if (!(det > 0.0f) || !(tr * tr <= 4e4f * det) || !(thr >= 0.0f)) return kAll;
@@ -135,12 +160,17 @@ __device__ __forceinline__ uint32_t patch_mask(float cx, float cy, float ca, flo
   const float hx = sqrtf(q * cc / det) * 1.05f + 0.25f;
   const float hy = sqrtf(q * ca / det) * 1.05f + 0.25f;
   if (!(hx < 1e30f) || !(hy < 1e30f)) return kAll;
+  if (f.axis != 0u && !single_image(f.axis == 1u ? hx : hy, f)) return kAll;
+  const float ccx = canonical_x(cx, f), ccy = canonical_y(cy, f);
   uint32_t m = 0;
 #pragma unroll
   for (uint32_t w = 0; w < (uint32_t)NW; ++w) {
     const float x0 = tile_x0 + (float)morton_compact(32u * w) + 0.5f;
     const float y0 = tile_y0 + (float)morton_compact(16u * w) + 0.5f;
-    const bool hit = cx + hx >= x0 && cx - hx <= x0 + 7.0f && cy + hy >= y0 && cy - hy <= y0 + 3.0f;
+    float px = cx, py = cy;
+    if (f.axis == 1u) px = ccx + nearest_image(ccx, x0 + 3.5f, f.vw) * f.vw;
+    if (f.axis == 2u) py = ccy + nearest_image(ccy, y0 + 1.5f, f.vh) * f.vh;
+    const bool hit = px + hx >= x0 && px - hx <= x0 + 7.0f && py + hy >= y0 && py - hy <= y0 + 3.0f;
     m |= hit ? (1u << w) : 0u;
   }
   return m;
@@ -203,7 +233,7 @@ __device__ __forceinline__ void blend_range(uint32_t begin, uint32_t source_coun
       sb.geo[t] = make_float4(m.x, m.y, m.w, thr);
       sb.con[t] = make_float4(c.x, c.y, c.z, m.z);
       sb.col[t] = __ldg(color + g);
-      sb.mask[t] = patch_mask<NT / 32>(m.x, m.y, c.x, c.y, c.z, thr, tile_x0, tile_y0, f.axis);
+      sb.mask[t] = patch_mask<NT / 32>(m.x, m.y, c.x, c.y, c.z, thr, tile_x0, tile_y0, f);
     }
     __syncthreads();
     const uint32_t n = min(NB, s1 - b);
