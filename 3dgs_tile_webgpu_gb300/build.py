@@ -1,9 +1,9 @@
 """Builds libgs3d.so (the C-ABI CUDA library) in-tree with nvcc for sm_103a.
 
-Translation units compile in parallel. ``pass_exact.cu`` holds every stage
-whose integer results must be bit-identical to the CPU restatement and
-``packer.cu`` restates the Rust packer's arithmetic; both are compiled with
-``--fmad=false``; the other units use the default contraction.
+Translation units compile in parallel. ``pass_exact.cu`` and ``front.cu`` hold
+every stage whose integer results must be bit-identical to the CPU restatement
+and ``packer.cu`` restates the Rust packer's arithmetic; these are compiled
+with ``--fmad=false``; the other units use the default contraction.
 """
 from __future__ import annotations
 
@@ -23,6 +23,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
           "-I", CSRC, "-I", INCLUDE]
 UNITS = {
     "pass_exact.cu": ["--fmad=false"],
+    "front.cu": ["--fmad=false"],
     "sort.cu": [],
     "raster.cu": [],
     "pipeline.cu": [],

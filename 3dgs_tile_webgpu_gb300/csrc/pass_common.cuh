@@ -54,8 +54,23 @@ struct PassOptions {
   uint32_t pixels_per_lane;  // fast raster forms: 2 (a warp per 8x8 patch) or 4 (per 8x16)
 };
 
-// The batch table in device memory: the per-frame parameters (attempt,
-// reset_valid), four ascending arrays (nviews + 1 entries each), then the view
+// The per-frame parameters at the head of a staged batch table. All but the
+// first two are the fused front's (front.cu), at their start values with every
+// copy: the range of the visible depth keys and the counters of its barriers,
+// each on an L2 line of its own (they are polled).
+enum FrameParam : uint32_t {
+  kFrameAttempt = 0,
+  kFrameReset = 1,
+  kFrameKeyMin = 2,
+  kFrameKeyMax = 3,
+  kFrameBarrier = 32,
+  kFrameDepthBarrier = 64,
+  kFrameTileBarrier = 96,
+  kFrameParams = 128
+};
+
+// The batch table in device memory: the per-frame parameters
+// (FrameParam), four ascending arrays (nviews + 1 entries each), then the view
 // descriptors. Consecutive views that render the same packed scene form a view
 // group, projected together (group_block: first projection block of each
 // group; group_view: first view of each group; ngroups + 1 entries used).
@@ -65,7 +80,7 @@ struct BatchView {
   const uint32_t* group_block;
   const uint32_t* group_view;
   const ViewDesc* views;
-  const uint32_t* frame_params;  // attempt, reset_valid
+  const uint32_t* frame_params;  // FrameParam
   uint32_t nviews;
   uint32_t ngroups;
   uint32_t total_items;
@@ -283,6 +298,23 @@ void launch_chunk_pass(int bits, const uint32_t* keys_in, const uint32_t* vals_i
 // Opt every sort-scatter instantiation into its shared-memory size (once per
 // device; call before any stream capture).
 void prepare_sort_kernels();
+// The fused front of small launches (front.cu): the stages before the
+// rasterizer in one cooperative kernel of kFrontBlocksPerSm blocks per SM at
+// most. front_fits: whether all of them are resident at once on the (current)
+// device. frame_params: the staged
+// table's FrameParam words on the device. tile_order null: no work list.
+constexpr uint32_t kFrontBlocksPerSm = 3;
+size_t front_scratch_words(int sms);  // words of FrontBuffers::scratch
+struct FrontBuffers {
+  float4 *mean, *conic, *color, *rec, *erec;
+  uint32_t *tile_counts, *keys, *vis_off, *dk[2], *dv[2], *ordered, *ioff, *tk[2], *tv[2];
+  uint32_t *tile_offsets, *tile_order, *scratch;
+  Control* ctl;
+  uint32_t* output_state;
+};
+bool front_fits(int device);
+void launch_front(const BatchView& b, const PassOptions& o, const FrontBuffers& w, uint32_t* frame_params,
+                  uint32_t capacity, uint32_t tile_passes, uint32_t digit_bits, int sms, cudaStream_t st);
 // Raster work list: every tile of the batch, heaviest load class first.
 void launch_tile_order(const uint32_t* tile_offsets, uint32_t ntile, Control* ctl, uint32_t* order, int sms,
                        cudaStream_t st);

@@ -63,8 +63,8 @@ __global__ void k_summary_add(BatchSummary* s, const Control* c, const uint32_t*
   for (int i = 0; i < 4; ++i) s->raster[i] += c->raster_stats[i];
   s->chunks += 1u;
   if (last) {
-    const uint32_t attempt = frame_params[0];
-    const uint32_t last_version = frame_params[1] ? 0u : s->prev_version;
+    const uint32_t attempt = frame_params[kFrameAttempt];
+    const uint32_t last_version = frame_params[kFrameReset] ? 0u : s->prev_version;
     output_state[0] = attempt;
     output_state[1] = s->overflow ? last_version : attempt;
     output_state[2] = s->requested;
@@ -79,6 +79,7 @@ struct gs3d_pipeline {
   gs3d_gaussian_data data{};
   int device = 0;
   int sms = 148;
+  bool front_ok = false;  // the fused front's blocks fit the device
   std::string error;
   // Per-slot workspaces (sized by data.count).
   uint32_t slot_cap = 0;
@@ -505,7 +506,8 @@ gs3d_status gs3d_pipeline_create(const gs3d_pipeline_desc* desc, const gs3d_gaus
   for (uint32_t i = 0; i < kObjectRing; ++i) cudaEventCreateWithFlags(&p->stage_ev[i], cudaEventDisableTiming);
   if ((e = dalloc(p->ctl, 1)) || (e = dalloc(p->output_state, 4)) || (e = dalloc(p->epoch_dev, 1)) ||
       (e = dalloc(p->summary, 1)) ||
-      (e = dalloc(p->chunk_counts, (size_t)kChunkBlocksPerSm * (size_t)p->sms * 256u))) {
+      (e = dalloc(p->chunk_counts,
+                  std::max((size_t)kChunkBlocksPerSm * (size_t)p->sms * 256u, front_scratch_words(p->sms))))) {
     s = cuda_fail(p, e, "allocating control block");
     release_all(p);
     delete p;
@@ -516,6 +518,7 @@ gs3d_status gs3d_pipeline_create(const gs3d_pipeline_desc* desc, const gs3d_gaus
   cudaMemset(p->epoch_dev, 0, sizeof(uint32_t));
   cudaMemset(p->summary, 0, sizeof(BatchSummary));
   prepare_sort_kernels();
+  p->front_ok = front_fits(p->device);
   if ((s = ensure_slots(p, data->count)) != GS3D_OK || (s = ensure_capacity(p, desc->intersection_capacity)) != GS3D_OK ||
       (s = ensure_stage(p, 16384)) != GS3D_OK) {
     release_all(p);
@@ -593,7 +596,7 @@ struct Plan {
 // rows: frame parameters and the four base arrays, view descriptors, object
 // rows.
 void layout_plan(Plan* pl, uint32_t n, size_t objects) {
-  const size_t header = 16 + align16(4 * (size_t)(n + 1) * sizeof(uint32_t));
+  const size_t header = kFrameParams * sizeof(uint32_t) + align16(4 * (size_t)(n + 1) * sizeof(uint32_t));
   pl->views_off = header;
   pl->objects_off = align16(header + (size_t)n * sizeof(ViewDesc));
   pl->stage_bytes = pl->objects_off + objects * 40 * sizeof(float);
@@ -671,10 +674,11 @@ void stage_batch(gs3d_pipeline* p, const gs3d_view* views, const Plan& pl, uint3
                  unsigned char* host, unsigned char* dev) {
   const uint32_t n = pl.n;
   uint32_t* params = (uint32_t*)host;
-  params[0] = attempt;
-  params[1] = reset_valid ? 1u : 0u;
-  params[2] = params[3] = 0u;
-  uint32_t* h_item = params + 4;
+  memset(params, 0, kFrameParams * sizeof(uint32_t));
+  params[kFrameAttempt] = attempt;
+  params[kFrameReset] = reset_valid ? 1u : 0u;
+  params[kFrameKeyMin] = 0xffffffffu;
+  uint32_t* h_item = params + kFrameParams;
   uint32_t* h_tile = h_item + (n + 1);
   uint32_t* h_gblock = h_tile + (n + 1);
   uint32_t* h_gview = h_gblock + (n + 1);
@@ -741,13 +745,30 @@ void stage_batch(gs3d_pipeline* p, const gs3d_view* views, const Plan& pl, uint3
   p->total_tiles = tile;
 }
 
+// Launches of up to this many ordinals take the fused front (front.cu): its
+// three blocks per SM project and sort slower than the separate kernels, but
+// it saves their launches. Frames of n ordinals at 1280x720 / 1920x1080, us,
+// front against separate kernels: 2k 69 / 164 and 78 / 176, 60k 93 / 187 and
+// 102 / 195, 200k 164 / 230 and 173 / 240, 400k 242 / 309 and 287 / 308 (with
+// a clustered scene 313 / 372 and 279 / 322), 520k 326 / 353 and 356 / 345,
+// 1M 549 / 484 and 551 / 487.
+constexpr uint32_t kFrontMaxItems = 3u << 17;
+
+// Profiled renders (events between the stages), the FP64 projection form, a
+// set wait limit and the withheld-chunk hook (both of the look-back waits,
+// which the front has none of) keep the separate kernels.
+bool use_front(const gs3d_pipeline* p, const Plan& pl) {
+  return p->front_ok && pl.items > 0 && pl.items <= kFrontMaxItems && !p->profiling &&
+         p->desc.projection_precision != GS3D_PROJECTION_FP64 && p->wait_limit == 0u && !p->withhold_first_chunk;
+}
+
 // Enqueue the pass over a staged batch table at `dev` (capturable: launches
 // and memsets only).
 void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStream_t st) {
   const uint32_t n = pl.n;
   BatchView bv;
   bv.frame_params = (const uint32_t*)dev;
-  bv.item_base = bv.frame_params + 4;
+  bv.item_base = bv.frame_params + kFrameParams;
   bv.tile_base = bv.item_base + (n + 1);
   bv.group_block = bv.tile_base + (n + 1);
   bv.group_view = bv.group_block + (n + 1);
@@ -784,6 +805,30 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
   const uint32_t tile = pl.tiles;
   uint32_t launches = 0;
   Control* ctl = p->ctl;
+  // Tile sort: fewest passes with digits of at most tuning.tile_digit_bits,
+  // then the narrowest digit; never more than the 4 passes the digit
+  // histograms hold (the digit then widens past the tuning, up to 8 bits for
+  // 32-bit ids).
+  const uint32_t cap32 = (uint32_t)p->capacity;
+  const uint32_t tile_bits = std::max(1u, ceil_log2((uint64_t)tile + 1));
+  const uint32_t max_digit = p->tuning.tile_digit_bits;
+  const int tile_passes = (int)std::min<uint32_t>(kMaxSortPasses, (tile_bits + max_digit - 1) / max_digit);
+  const int digit_bits = (int)((tile_bits + tile_passes - 1) / tile_passes);
+  const bool exact = p->desc.raster_precision == GS3D_RASTER_EXACT;
+  const bool ordered_tiles = p->tuning.work_order != 0u;
+  if (use_front(p, pl)) {
+    const FrontBuffers w = {p->mean, p->conic, p->color, exact ? nullptr : p->rec, p->erec, p->counts, p->keys,
+                            p->vis_off, {p->dk[0], p->dk[1]}, {p->dv[0], p->dv[1]}, p->ordered, p->ioff,
+                            {p->tk[0], p->tk[1]}, {p->tv[0], p->tv[1]}, p->tile_offsets,
+                            ordered_tiles ? p->tile_order : nullptr, p->chunk_counts, ctl, p->output_state};
+    launch_front(bv, o, w, (uint32_t*)dev, cap32, (uint32_t)tile_passes, (uint32_t)digit_bits, p->sms, st);
+    p->depth_final = 0;
+    p->tile_final = tile_passes & 1;
+    launch_raster((int)p->desc.raster_precision, p->tile_offsets, w.tile_order, p->tv[p->tile_final], p->mean,
+                  p->conic, p->color, p->rec, bv, o, ctl, p->desc.raster_stats != 0, st);
+    p->last_launches = 2;
+    return;
+  }
   uint32_t ep = 0;  // look-back launch index within the frame
   auto epoch = [&]() { return Epoch{p->epoch_dev, ++ep, p->wait_limit}; };
   launch_epoch_begin(p->epoch_dev, st);
@@ -800,7 +845,6 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
 
   // K1: projection.
   mark(p, GS3D_STAGE_PROJECT, st);
-  const bool exact = p->desc.raster_precision == GS3D_RASTER_EXACT;
   launch_project(bv, o, p->mean, p->conic, p->color, p->counts, p->keys, exact ? nullptr : p->rec, p->erec, st);
   launches += pl.blocks ? 1 : 0;
   // Visibility compaction.
@@ -822,19 +866,11 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
   p->depth_final = cur;
   // Ordered counts + saturating scan + dispatch/output state.
   mark(p, GS3D_STAGE_SCAN, st);
-  const uint32_t cap32 = (uint32_t)p->capacity;
   launch_scan_counts(p->dv[cur], p->counts, p->ordered, p->ioff, ctl, p->status, epoch(), cap32, bv.frame_params,
                      p->output_state, scan_grid, st);
   ++launches;
   // Emission + tile-sort histograms.
   mark(p, GS3D_STAGE_EMIT, st);
-  // Fewest passes with digits of at most tuning.tile_digit_bits, then the
-  // narrowest digit; never more than the 4 passes the digit histograms hold
-  // (the digit then widens past the tuning, up to 8 bits for 32-bit ids).
-  const uint32_t tile_bits = std::max(1u, ceil_log2((uint64_t)tile + 1));
-  const uint32_t max_digit = p->tuning.tile_digit_bits;
-  const int tile_passes = (int)std::min<uint32_t>(kMaxSortPasses, (tile_bits + max_digit - 1) / max_digit);
-  const int digit_bits = (int)((tile_bits + tile_passes - 1) / tile_passes);
   launch_emit(p->dv[cur], N, p->erec, p->ordered, p->ioff, bv, o, ctl, cap32, p->tk[0], p->tv[0], st);
   launches += N ? 1 : 0;
   // Tile sort.
@@ -852,7 +888,6 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
   mark(p, GS3D_STAGE_RANGES, st);
   launch_tile_ranges(p->tk[tcur], ctl, tile, cap32, p->tile_offsets, st);
   ++launches;
-  const bool ordered_tiles = p->tuning.work_order != 0u;
   if (ordered_tiles) {
     launch_tile_order(p->tile_offsets, tile, ctl, p->tile_order, p->sms, st);
     launches += 2;

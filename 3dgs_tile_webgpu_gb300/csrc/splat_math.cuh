@@ -207,7 +207,7 @@ __device__ __forceinline__ Projected project(f3 view, const m3& cv, const float*
 // translation) and for near-singular splats (the 2D covariance, its
 // determinant and the conic lose most of their bits in FP32 when the
 // projected covariance is nearly rank one).
-__device__ __noinline__ Projected project_fp64(double vx, double vy, double vz, float4 so, float4 q_in,
+static __device__ __noinline__ Projected project_fp64(double vx, double vy, double vz, float4 so, float4 q_in,
                                                const float* mv, const float* P, float vw, float vh, float vnear,
                                                float vfar, float filter) {
   Projected o;
