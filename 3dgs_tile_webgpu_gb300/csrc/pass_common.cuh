@@ -111,7 +111,7 @@ struct Control {
   uint32_t tile_hist[kMaxSortPasses][256];   // digit histograms of the tile sort (its count kernels)
   uint32_t visible_state[4];     // visible, visible, radix blocks, 0
   uint32_t state[4];             // count, total, radix blocks, overflow
-  uint32_t error;                // bit 0: look-back wait expired; bit 2: a sort tile copy never landed
+  uint32_t error;                // bit 0: look-back wait or grid barrier expired; bit 2: a sort tile copy never landed
   uint32_t pad[3];
   unsigned long long raster_stats[4];  // checked, blended, pixels, alpha-stopped
   uint32_t order_hist[34];       // raster work-list buckets (tile load classes)

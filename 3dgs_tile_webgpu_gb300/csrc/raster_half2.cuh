@@ -192,30 +192,42 @@ __device__ __forceinline__ void blend_range_h2(uint32_t begin, uint32_t source_c
     if (capped) src = (uint32_t)floorf((((float)i + 0.5f) * (float)source_count) / (float)raster_count);
     return __ldg(ids + begin + src);
   };
-  // The FP32 form loads the next group's record ids one group ahead (the
-  // half2 form, at its register limit for 10 blocks per SM, is faster without).
-  uint32_t next_id = HALF ? 0u : load_id(s0 + lane);
+  // The half2 form gathers the next group's records before it blends this
+  // one's; the FP32 form, at its register limit, loads their ids only.
+  uint32_t next_id = load_id(s0 + lane);
+  float4 n0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), n1 = n0;
+  float next_depth = 0.0f;
+  auto gather = [&](uint32_t i, uint32_t g) {
+    if (i >= s1) return;
+    n0 = __ldg(rec + 2 * (size_t)g);  // one 32-byte record
+    n1 = __ldg(rec + 2 * (size_t)g + 1);
+    if (DEPTH && need_depth) next_depth = __ldg(&mean[g].z);
+  };
+  if (HALF) {
+    gather(s0 + lane, next_id);
+    next_id = load_id(s0 + 32u + lane);
+  }
   for (uint32_t b = s0; b < s1; b += 32) {
     if (__all_sync(0xffffffffu, done0 && done1)) break;
     const uint32_t i = b + lane;
     bool reach = false;
-    float4 r0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), r1 = r0, col32 = r0;
-    float depth = 0.0f, image = 0.0f;
-    uint32_t cur_id = 0;
-    if (!HALF) {
-      cur_id = next_id;
+    float4 r0, r1, col32 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float depth, image = 0.0f;
+    if (HALF) {
+      r0 = n0; r1 = n1; depth = next_depth;
+      gather(b + 32u + lane, next_id);
+      next_id = load_id(b + 64u + lane);
+    } else {
+      const uint32_t g = next_id;
       next_id = load_id(b + 32u + lane);
+      gather(i, g);
+      r0 = n0; r1 = n1; depth = next_depth;
+      if (i < s1) col32 = __ldg(color + g);
     }
-    if (i < s1) {
-      const uint32_t g = HALF ? load_id(i) : cur_id;
-      r0 = __ldg(rec + 2 * (size_t)g);  // one 32-byte record
-      r1 = __ldg(rec + 2 * (size_t)g + 1);
-      if (!HALF) col32 = __ldg(color + g);
-      if (DEPTH && need_depth) depth = __ldg(&mean[g].z);
+    if (i < s1)
       reach = PERIODIC ? periodic_reach(r0, r1, f, patch_x0 + 0.5f, patch_y0 + 0.5f, 7.0f, 7.0f, &image)
                        : patch_reach(r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, patch_x0 + 0.5f, patch_y0 + 0.5f, 7.0f,
                                      7.0f);
-    }
     const uint32_t bal = __ballot_sync(0xffffffffu, reach);
     if (reach) {
       const uint32_t q = __popc(bal & lt);
@@ -592,13 +604,18 @@ template <int TILE>
 constexpr int h2_threads() {
   return 32 * (TILE / 8) * (TILE / 8);
 }
-// Resident blocks per SM the register budget is set for: 10 blocks of 128
-// threads (half2: 48 registers; 9 and 12 blocks measured slower) / 8 (FP32)
-// at the reference's 16-pixel tiles, the same threads per SM at other tile
-// sizes (at most 32 blocks).
+// Resident blocks per SM the register budget is set for: 9 blocks of 128
+// threads (half2: 56 registers, which hold the next group's records) / 8
+// (FP32: 64) at the reference's 16-pixel tiles, the same threads per SM at
+// other tile sizes (at most 32 blocks). Rasterizer, us: half2 without the
+// prefetch at 10 / 9 blocks, with it at 9 / 8: 16 views of 3M splats at 1080p
+// 3103 / 3157 / 3129 / 3284, four mixed views of 500k splats 368 / 356 / 294 /
+// 296 (its heaviest tile holds 6768 records, the mean 246: a warp's walk of
+// one list is the bound there). FP32 with the prefetch at 7 blocks: 3M splats
+// at 1080p 350 -> 336, eight objects in eight views 1601 -> 1629; not taken.
 template <bool HALF, int TILE>
 constexpr int h2_min_blocks() {
-  return (HALF ? 1280 : 1024) / h2_threads<TILE>() > 32 ? 32 : (HALF ? 1280 : 1024) / h2_threads<TILE>();
+  return (HALF ? 1152 : 1024) / h2_threads<TILE>() > 32 ? 32 : (HALF ? 1152 : 1024) / h2_threads<TILE>();
 }
 
 template <bool HALF, bool PERIODIC, bool STATS, bool DEPTH, int TILE>
