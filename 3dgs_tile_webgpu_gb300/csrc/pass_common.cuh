@@ -107,8 +107,8 @@ uint32_t scan_chunks(uint32_t n_max, int sms);
 // Per-frame control block, zeroed before each render.
 struct Control {
   uint32_t tickets[2];           // dynamic tile ids of the look-back kernels (Ticket)
-  uint32_t depth_hist[kMaxSortPasses][256];  // digit histograms of the depth sort (its count kernels)
-  uint32_t tile_hist[kMaxSortPasses][256];   // digit histograms of the tile sort (its count kernels)
+  uint32_t depth_hist[kMaxSortPasses][256];  // digit histograms of the fused front's chunked passes:
+  uint32_t tile_hist[kMaxSortPasses][256];   // depth sort and tile sort
   uint32_t visible_state[4];     // visible, visible, radix blocks, 0
   uint32_t state[4];             // count, total, radix blocks, overflow
   uint32_t error;                // bit 0: look-back wait or grid barrier expired; bit 2: a sort tile copy never landed
@@ -125,7 +125,7 @@ enum Ticket { kTicketCompact = 0, kTicketScan = 1 };
 // A word whose epoch differs from the launch's epoch is "not yet published",
 // so the status array never needs clearing between launches. A frame's
 // launches use epochs base + 1 .. base + kEpochsPerFrame, where base is a
-// device-side counter advanced by k_epoch_begin at the start of every frame,
+// device-side counter advanced by k_frame_begin at the start of every frame,
 // so a replayed CUDA graph never reuses an epoch.
 constexpr uint32_t kEpochsPerFrame = 16;
 
@@ -267,7 +267,9 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
 // (conic c, log(opacity * 255), rx + 512 ry, 0), written for visible items.
 void launch_project(const BatchView& b, const PassOptions& o, float4* mean, float4* conic, float4* color,
                     uint32_t* counts, uint32_t* keys, float4* rec, float4* erec, cudaStream_t st);
-void launch_epoch_begin(uint32_t* epoch_base, cudaStream_t st);
+// Starts a frame: advances the look-back epoch and clears `words` words (the
+// sorts' sums and the control block).
+void launch_frame_begin(uint32_t* epoch_base, uint32_t* zero, uint32_t words, cudaStream_t st);
 // Advance ticket counter `ticket` of the control block by one (a test hook:
 // the chunk of ticket 0 is then never scanned, so its successor's look-back
 // wait runs out).
@@ -284,17 +286,20 @@ void launch_emit(const uint32_t* sorted_ids, uint32_t n_max, const float4* erec,
 void launch_tile_ranges(const uint32_t* sorted_tile_keys, Control* ctl, uint32_t ntile, uint32_t n_max,
                         uint32_t* tile_offsets, cudaStream_t st);
 constexpr uint32_t kSortTile = 4096;  // items per sort tile
-// Chunked LSD pass (reduce, scan, scatter; no look-back chain): `chunks`
-// blocks, each walking a contiguous run of 4096-item tiles. counts holds
-// chunks x 2^bits words; hist (2^bits words, zero on entry) receives the
-// pass's digit histogram. n is read from *n_ptr on the device.
+// Chunked LSD pass (reduce, scatter; no look-back chain): `chunks` blocks,
+// each walking a contiguous run of 4096-item tiles. counts holds chunks rows
+// of 2^bits words; sums (sum_rows(chunks) rows of 256 words, zero on entry)
+// takes the counts of 16 chunks a row; spare, as large, is zeroed (the next
+// pass takes it as its sums). n is read from *n_ptr on the device.
 constexpr uint32_t kChunkBlocksPerSm = 3;
+constexpr uint32_t kSumChunks = 16;
+constexpr uint32_t sum_rows(uint32_t chunks) { return (chunks + kSumChunks - 1u) / kSumChunks; }
 uint32_t chunk_pass_chunks(uint32_t n_max, int sms);
 // err: the control block's error word (bit 2: a tile copy of the scatter
 // never landed).
 void launch_chunk_pass(int bits, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
-                       uint32_t* vals_out, const uint32_t* n_ptr, int shift, uint32_t* hist, uint32_t chunks,
-                       uint32_t* counts, uint32_t* err, cudaStream_t st);
+                       uint32_t* vals_out, const uint32_t* n_ptr, int shift, uint32_t chunks, uint32_t* counts,
+                       uint32_t* sums, uint32_t* spare, uint32_t* err, cudaStream_t st);
 // Opt every sort-scatter instantiation into its shared-memory size (once per
 // device; call before any stream capture).
 void prepare_sort_kernels();

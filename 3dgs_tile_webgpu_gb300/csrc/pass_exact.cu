@@ -192,13 +192,18 @@ __global__ void __launch_bounds__(kBlock) k_compact(const uint32_t* __restrict__
   }
 }
 
-__global__ void k_epoch_begin(uint32_t* base) {
+__global__ void __launch_bounds__(kBlock) k_frame_begin(uint32_t* base, uint32_t* __restrict__ zero,
+                                                        uint32_t words) {
+  for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < words; i += gridDim.x * kBlock) zero[i] = 0u;
+  if (blockIdx.x != 0 || threadIdx.x != 0) return;
   // Leaves room for kEpochsPerFrame launches; status words are 30-bit epochs.
   const uint32_t next = (*base + kEpochsPerFrame) & ((1u << 30) - 1u);
   *base = next < kEpochsPerFrame ? kEpochsPerFrame : next;
 }
 
-void launch_epoch_begin(uint32_t* epoch_base, cudaStream_t st) { k_epoch_begin<<<1, 1, 0, st>>>(epoch_base); }
+void launch_frame_begin(uint32_t* epoch_base, uint32_t* zero, uint32_t words, cudaStream_t st) {
+  k_frame_begin<<<(words + kBlock * 4u - 1u) / (kBlock * 4u), kBlock, 0, st>>>(epoch_base, zero, words);
+}
 
 __global__ void k_skip_ticket(Control* ctl, uint32_t ticket) { ctl->tickets[ticket] += 1u; }
 

@@ -110,6 +110,10 @@ struct gs3d_pipeline {
   size_t status_words = 0;
   // Per-(chunk, digit) counts of the chunked sort passes.
   uint32_t* chunk_counts = nullptr;
+  // Cleared at the start of a frame: the chunked passes' two sets of sums,
+  // then the control block (ctl).
+  uint32_t* zeroed = nullptr;
+  uint32_t sum_words = 0;  // words of one set of sums
   uint32_t epoch = 0;
   // Batch-table staging (bases, view descriptors, object tables), a ring of
   // pinned host buffers each mirrored by a device buffer.
@@ -436,7 +440,7 @@ void release_all(gs3d_pipeline* p) {
   dfree(p->mean); dfree(p->rec); dfree(p->erec); dfree(p->conic); dfree(p->color); dfree(p->counts); dfree(p->keys); dfree(p->vis_off);
   dfree(p->dk[0]); dfree(p->dk[1]); dfree(p->dv[0]); dfree(p->dv[1]); dfree(p->ordered); dfree(p->ioff);
   dfree(p->tk[0]); dfree(p->tk[1]); dfree(p->tv[0]); dfree(p->tv[1]);
-  dfree(p->tile_offsets); dfree(p->tile_order); dfree(p->ctl); dfree(p->epoch_dev); dfree(p->output_state); dfree(p->status);
+  dfree(p->tile_offsets); dfree(p->tile_order); dfree(p->zeroed); dfree(p->epoch_dev); dfree(p->output_state); dfree(p->status);
   dfree(p->chunk_counts);
   dfree(p->summary); dfree(p->profile_sums); dfree(p->profile_hist); dfree(p->profile_zero);
 }
@@ -504,7 +508,9 @@ gs3d_status gs3d_pipeline_create(const gs3d_pipeline_desc* desc, const gs3d_gaus
   }
   cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
   for (uint32_t i = 0; i < kObjectRing; ++i) cudaEventCreateWithFlags(&p->stage_ev[i], cudaEventDisableTiming);
-  if ((e = dalloc(p->ctl, 1)) || (e = dalloc(p->output_state, 4)) || (e = dalloc(p->epoch_dev, 1)) ||
+  p->sum_words = sum_rows(kChunkBlocksPerSm * (uint32_t)p->sms) * 256u;
+  if ((e = dalloc(p->zeroed, 2 * (size_t)p->sum_words + sizeof(Control) / sizeof(uint32_t))) ||
+      (e = dalloc(p->output_state, 4)) || (e = dalloc(p->epoch_dev, 1)) ||
       (e = dalloc(p->summary, 1)) ||
       (e = dalloc(p->chunk_counts,
                   std::max((size_t)kChunkBlocksPerSm * (size_t)p->sms * 256u, front_scratch_words(p->sms))))) {
@@ -513,6 +519,7 @@ gs3d_status gs3d_pipeline_create(const gs3d_pipeline_desc* desc, const gs3d_gaus
     delete p;
     return s;
   }
+  p->ctl = (Control*)(p->zeroed + 2 * (size_t)p->sum_words);
   cudaMemset(p->output_state, 0, 4 * sizeof(uint32_t));
   cudaMemset(p->ctl, 0, sizeof(Control));
   cudaMemset(p->epoch_dev, 0, sizeof(uint32_t));
@@ -831,9 +838,11 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
   }
   uint32_t ep = 0;  // look-back launch index within the frame
   auto epoch = [&]() { return Epoch{p->epoch_dev, ++ep, p->wait_limit}; };
-  launch_epoch_begin(p->epoch_dev, st);
-  cudaMemsetAsync(ctl, 0, sizeof(Control), st);
+  launch_frame_begin(p->epoch_dev, p->zeroed, 2u * p->sum_words + (uint32_t)(sizeof(Control) / sizeof(uint32_t)), st);
   launches += 1;
+  // The sort passes take turns with the two sets of sums.
+  uint32_t* sums = p->zeroed;
+  uint32_t* spare = p->zeroed + p->sum_words;
   if (p->withhold_first_chunk) {
     // Test hook (gs3d_pipeline_debug_withhold_chunk): the compaction's ticket
     // counter starts at 1, so no block scans chunk 0 and the look-back of
@@ -859,9 +868,10 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
   const uint32_t depth_chunks = chunk_pass_chunks(N, p->sms);
   for (int pass = 0; pass < depth_passes; ++pass) {
     launch_chunk_pass(8, p->dk[cur], p->dv[cur], p->dk[cur ^ 1], p->dv[cur ^ 1], &ctl->visible_state[0], 8 * pass,
-                      ctl->depth_hist[pass], depth_chunks, p->chunk_counts, &ctl->error, st);
+                      depth_chunks, p->chunk_counts, sums, spare, &ctl->error, st);
+    std::swap(sums, spare);
     cur ^= 1;
-    launches += 3;
+    launches += 2;
   }
   p->depth_final = cur;
   // Ordered counts + saturating scan + dispatch/output state.
@@ -879,9 +889,10 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
   const uint32_t tile_chunks = chunk_pass_chunks(cap32, p->sms);
   for (int pass = 0; pass < tile_passes; ++pass) {
     launch_chunk_pass(digit_bits, p->tk[tcur], p->tv[tcur], p->tk[tcur ^ 1], p->tv[tcur ^ 1], &ctl->state[0],
-                      digit_bits * pass, ctl->tile_hist[pass], tile_chunks, p->chunk_counts, &ctl->error, st);
+                      digit_bits * pass, tile_chunks, p->chunk_counts, sums, spare, &ctl->error, st);
+    std::swap(sums, spare);
     tcur ^= 1;
-    launches += 3;
+    launches += 2;
   }
   p->tile_final = tcur;
   // Tile ranges and the raster work list.

@@ -10,12 +10,18 @@
 // decoupled look-back pass settles only a window of tiles per L2 round trip,
 // which bounds it far below HBM speed on passes of tens of millions of keys).
 // The items split into `chunks` contiguous runs of whole 4096-item tiles (one
-// split, derived from the device-side count, shared by the three kernels):
-//   k_chunk_count   keys of every (chunk, digit), by shared-memory atomics,
-//                   also summed into the pass's global digit histogram;
-//   k_chunk_offsets per digit, the exclusive prefix over chunks plus the
-//                   digit's global base from that histogram;
-//   k_chunk_scatter one block per chunk walks its tiles in order with running
+// split, derived from the device-side count, shared by the two kernels; the
+// runs differ by at most one tile, so that no SM gets two tiles more than
+// another: with runs of ceil(tiles / chunks), 2.3M items kept 280 of the 456
+// blocks busy):
+//   k_chunk_count   keys of every (chunk, digit), by shared-memory atomics:
+//                   a row of counts per chunk, and rows of sums over 16
+//                   chunks each, added up by atomics;
+//   k_chunk_scatter one block per chunk adds up the sums of the
+//                   groups of chunks before its own and the rows before its
+//                   own in its group (at most 29 + 15 rows; a kernel between
+//                   the two that turned the counts into positions took 6 us a
+//                   pass), then walks its tiles in order with running
 //                   per-digit offsets: tile t+1 streams into shared memory by
 //                   two bulk copies (cp.async.bulk, 16 KB of keys and 16 KB
 //                   of values, completion counted on an mbarrier) while tile
@@ -26,6 +32,13 @@
 //                   written out with each digit's run contiguous.
 // Stable: tiles in index order within a chunk, chunks in index order, ranks in
 // index order within a tile.
+// Bound by instructions and shared memory (ballots, one look-up and two random
+// stores per item), not by HBM. us, with offsets kernel, equal chunk sizes and
+// two look-ups -> so: depth sort of 2.3M / 6M / 2 x 17.5M items 156 -> 122,
+// 253 -> 208, 1125 -> 1087; tile sort of 5.5M / 17.7M / 2 x 42.7M / 398M
+// records 97 -> 83, 252 -> 229, 1252 -> 1199, 5433 -> 5286 (2.4 TB/s of
+// scattered writes and reads). 512 threads of 8 items spill at 40 registers:
+// 1201 and 1323 for the 16 views.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -35,8 +48,11 @@
 
 namespace gs {
 
-constexpr int kSortWarps = 8;
+constexpr int kCountWarps = kBlock / 32;
+constexpr int kScatterThreads = 256;
+constexpr int kSortWarps = kScatterThreads / 32;
 constexpr int kSortItems = 16;  // kSortTile = 8 warps * 32 lanes * 16 items
+static_assert(kSortTile == (uint32_t)(kScatterThreads * kSortItems), "a tile is 16 items per thread");
 
 // Lanes of the warp holding the same BITS-bit digit, by ballot bit-splitting.
 template <int BITS>
@@ -54,21 +70,20 @@ __device__ __forceinline__ uint32_t match_digit(uint32_t d, uint32_t valid_mask)
 // Tiles [t0, t1) of chunk c when n items split over `chunks` chunks.
 __device__ __forceinline__ void chunk_tiles(uint32_t n, uint32_t chunks, uint32_t c, uint32_t* t0, uint32_t* t1) {
   const uint32_t tiles = (uint32_t)(((uint64_t)n + kSortTile - 1) / kSortTile);
-  const uint32_t per = (tiles + chunks - 1) / chunks;
-  *t0 = min(c * per, tiles);
-  *t1 = min(*t0 + per, tiles);
+  *t0 = (uint32_t)((uint64_t)c * tiles / chunks);
+  *t1 = (uint32_t)((uint64_t)(c + 1u) * tiles / chunks);
 }
 
 template <int BITS>
 __global__ void __launch_bounds__(kBlock) k_chunk_count(const uint32_t* __restrict__ keys,
                                                         const uint32_t* __restrict__ n_ptr, int shift,
                                                         uint32_t chunks, uint32_t* __restrict__ counts,
-                                                        uint32_t* __restrict__ hist) {
+                                                        uint32_t* __restrict__ sums) {
   constexpr uint32_t RADIX = 1u << BITS;
   constexpr uint32_t MASK = RADIX - 1u;
-  __shared__ uint32_t s_hist[kSortWarps][RADIX];
+  __shared__ uint32_t s_hist[kCountWarps][RADIX];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  for (uint32_t i = tid; i < kSortWarps * RADIX; i += kBlock) (&s_hist[0][0])[i] = 0u;
+  for (uint32_t i = tid; i < kCountWarps * RADIX; i += kBlock) (&s_hist[0][0])[i] = 0u;
   __syncthreads();
   const uint32_t n = *n_ptr;
   uint32_t t0, t1;
@@ -78,7 +93,7 @@ __global__ void __launch_bounds__(kBlock) k_chunk_count(const uint32_t* __restri
   // Each warp takes 512-key runs: four 16-byte loads per lane in flight
   // before any counting (begin is a multiple of 4096, so they are aligned).
   constexpr uint32_t kRun = 512u;
-  for (uint32_t s = begin + warp * kRun; s < end; s += kSortWarps * kRun) {
+  for (uint32_t s = begin + warp * kRun; s < end; s += kCountWarps * kRun) {
     uint32_t kk[16];
 #pragma unroll
     for (uint32_t q = 0; q < 4u; ++q) {
@@ -107,32 +122,9 @@ __global__ void __launch_bounds__(kBlock) k_chunk_count(const uint32_t* __restri
   for (uint32_t d = tid; d < RADIX; d += kBlock) {
     uint32_t sum = 0;
 #pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) sum += s_hist[w][d];
+    for (int w = 0; w < kCountWarps; ++w) sum += s_hist[w][d];
     counts[(size_t)blockIdx.x * RADIX + d] = sum;
-    if (sum) atomicAdd(hist + d, sum);
-  }
-}
-
-// One block per digit; counts[c][d] becomes the global position of the first
-// key of digit d in chunk c.
-template <int BITS>
-__global__ void __launch_bounds__(kBlock) k_chunk_offsets(const uint32_t* __restrict__ hist, uint32_t chunks,
-                                                          uint32_t* __restrict__ counts) {
-  constexpr uint32_t RADIX = 1u << BITS;
-  __shared__ uint32_t s_scan[kBlock / 32];
-  const uint32_t tid = threadIdx.x, d = blockIdx.x;
-  uint32_t base;
-  block_exclusive_scan<false>(tid < d ? hist[tid] : 0u, s_scan, &base);  // keys of the digits below d
-  const uint32_t per = (chunks + kBlock - 1) / kBlock;
-  const uint32_t c0 = min(tid * per, chunks), c1 = min(c0 + per, chunks);
-  uint32_t local = 0;
-  for (uint32_t c = c0; c < c1; ++c) local += counts[(size_t)c * RADIX + d];
-  uint32_t total;
-  uint32_t run = base + block_exclusive_scan<false>(local, s_scan, &total);
-  for (uint32_t c = c0; c < c1; ++c) {
-    const uint32_t v = counts[(size_t)c * RADIX + d];
-    counts[(size_t)c * RADIX + d] = run;
-    run += v;
+    if (sum) atomicAdd(sums + blockIdx.x / kSumChunks * RADIX + d, sum);
   }
 }
 
@@ -142,12 +134,29 @@ constexpr size_t kChunkDynSmem = 2 * 2 * kSortTile * sizeof(uint32_t);
 
 template <int BITS>
 struct ScatterShared {
-  uint32_t warp_hist[kSortWarps][1u << BITS];
-  uint32_t block_excl[1u << BITS];
-  uint32_t run[1u << BITS];  // global position of the next key of each digit
-  uint32_t scan[kBlock / 32];
+  uint16_t warp_hist[kSortWarps][1u << BITS];  // a warp's items per digit, then its first tile position
+  uint32_t delta[1u << BITS];  // global position of the tile's item i of a digit, minus i
+  uint32_t scan[8];
   unsigned long long bar[2];  // bulk-copy completion of each tile buffer
 };
+
+// Exclusive scan of one value per digit over the threads below 256, in two
+// block barriers; every thread of the block calls it.
+__device__ __forceinline__ uint32_t digit_scan(uint32_t v, uint32_t* s_scan) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  if (lane == 31u && warp < 8u) s_scan[warp] = x;
+  __syncthreads();
+  uint32_t before = 0;
+#pragma unroll
+  for (uint32_t w = 0; w < 7u; ++w) before += w < warp ? s_scan[w] : 0u;
+  return before + x - v;
+}
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -175,7 +184,7 @@ __device__ __forceinline__ void load_tile_bulk(const uint32_t* __restrict__ keys
                    : "memory");
     }
   }
-  for (uint32_t e = whole + threadIdx.x; e < items; e += kBlock) {
+  for (uint32_t e = whole + threadIdx.x; e < items; e += kScatterThreads) {
     kb[e] = keys_in[base + e];
     vb[e] = vals_in[base + e];
   }
@@ -200,12 +209,13 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
 
 // Ranks the tile held in kb/vb (items base .. base + 4096, those below n),
 // stages it in place in block-sorted order and writes each digit's run to its
-// global position. FULL: every item of the tile is below n. Leaves warp_hist
-// zeroed and run advanced past the tile.
+// global position. FULL: every item of the tile is below n. `run`: the global
+// position of the next item of digit threadIdx.x (threads below 2^BITS).
+// Leaves warp_hist zeroed and run advanced past the tile.
 template <int BITS, bool FULL>
 __device__ __forceinline__ void scatter_tile(ScatterShared<BITS>& sm, uint32_t* kb, uint32_t* vb, uint32_t base,
                                              uint32_t n, int shift, uint32_t* __restrict__ keys_out,
-                                             uint32_t* __restrict__ vals_out) {
+                                             uint32_t* __restrict__ vals_out, uint32_t& run) {
   constexpr uint32_t RADIX = 1u << BITS;
   constexpr uint32_t MASK = RADIX - 1u;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -225,83 +235,108 @@ __device__ __forceinline__ void scatter_tile(ScatterShared<BITS>& sm, uint32_t* 
     if (ok) cnt = sm.warp_hist[warp][d];
     rank[j] = cnt + before;
     __syncwarp();
-    if (ok && before == 0) sm.warp_hist[warp][d] = cnt + __popc(peers);
+    if (ok && before == 0) sm.warp_hist[warp][d] = (uint16_t)(cnt + __popc(peers));
     __syncwarp();
   }
   __syncthreads();
 
-  uint32_t block_count = 0;
+  // Thread d: the tile's items of digit d, and with the digits below it the
+  // tile position of each warp's first item of digit d (one look-up per item
+  // below).
+  uint32_t count = 0;
   if (tid < RADIX) {
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) count += sm.warp_hist[w][tid];
+  }
+  const uint32_t excl = digit_scan(count, sm.scan);
+  if (tid < RADIX) {
+    uint32_t first = excl;
 #pragma unroll
     for (int w = 0; w < kSortWarps; ++w) {
       const uint32_t c = sm.warp_hist[w][tid];
-      sm.warp_hist[w][tid] = block_count;
-      block_count += c;
+      sm.warp_hist[w][tid] = (uint16_t)first;
+      first += c;
     }
-  }
-  {
-    uint32_t tot;
-    const uint32_t e = block_exclusive_scan<false>(tid < RADIX ? block_count : 0u, sm.scan, &tot);
-    if (tid < RADIX) sm.block_excl[tid] = e;
+    sm.delta[tid] = run - excl;
+    run += count;
   }
   __syncthreads();
 
-  // Keys first (every raw key is already in registers), then the values
-  // (read raw into registers, then written once every thread has read).
+  // Keys first (every raw key is in registers), then the values (read raw
+  // into the keys' registers, then written once every thread has read).
 #pragma unroll
   for (int j = 0; j < kSortItems; ++j) {
     if (FULL || base + wofs + (uint32_t)j * 32u + lane < n) {
       const uint32_t d = (k[j] >> shift) & MASK;
-      rank[j] += sm.block_excl[d] + sm.warp_hist[warp][d];
+      rank[j] += sm.warp_hist[warp][d];
       kb[rank[j]] = k[j];
     }
   }
-  uint32_t v[kSortItems];
 #pragma unroll
-  for (int j = 0; j < kSortItems; ++j) v[j] = vb[wofs + (uint32_t)j * 32u + lane];
+  for (int j = 0; j < kSortItems; ++j) k[j] = vb[wofs + (uint32_t)j * 32u + lane];
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < kSortItems; ++j)
-    if (FULL || base + wofs + (uint32_t)j * 32u + lane < n) vb[rank[j]] = v[j];
+    if (FULL || base + wofs + (uint32_t)j * 32u + lane < n) vb[rank[j]] = k[j];
   __syncthreads();
 
-  const uint32_t count = FULL ? kSortTile : min(kSortTile, n - base);
+  const uint32_t items = FULL ? kSortTile : min(kSortTile, n - base);
 #pragma unroll 4
-  for (uint32_t i = tid; i < count; i += kBlock) {
+  for (uint32_t i = tid; i < items; i += kScatterThreads) {
     const uint32_t key = kb[i];
-    const uint32_t dig = (key >> shift) & MASK;
-    const uint32_t dst = sm.run[dig] + (i - sm.block_excl[dig]);
+    const uint32_t dst = sm.delta[(key >> shift) & MASK] + i;
     keys_out[dst] = key;
     vals_out[dst] = vb[i];
   }
-  for (uint32_t i = tid; i < kSortWarps * RADIX; i += kBlock) (&sm.warp_hist[0][0])[i] = 0u;
+  for (uint32_t i = tid; i < kSortWarps * RADIX * sizeof(uint16_t) / 4u; i += kScatterThreads)
+    reinterpret_cast<uint32_t*>(&sm.warp_hist[0][0])[i] = 0u;
   __syncthreads();
-  if (tid < RADIX) sm.run[tid] += block_count;
 }
 
 template <int BITS>
-__global__ void __launch_bounds__(kBlock, kChunkBlocksPerSm)
+__global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
     k_chunk_scatter(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                     uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
                     const uint32_t* __restrict__ n_ptr, int shift, uint32_t chunks,
-                    const uint32_t* __restrict__ offsets, uint32_t* __restrict__ err) {
+                    const uint32_t* __restrict__ counts, const uint32_t* __restrict__ sums,
+                    uint32_t* __restrict__ spare, uint32_t* __restrict__ err) {
   constexpr uint32_t RADIX = 1u << BITS;
-  __shared__ ScatterShared<BITS> sm;
+  __shared__ __align__(16) ScatterShared<BITS> sm;
   extern __shared__ uint4 s_dyn[];
   uint32_t* s_buf = reinterpret_cast<uint32_t*>(s_dyn);
 
-  const uint32_t tid = threadIdx.x;
+  const uint32_t tid = threadIdx.x, c = blockIdx.x;
+  // The other sums, used by the pass before this one, start the next at zero.
+  if (c < (chunks + kSumChunks - 1u) / kSumChunks && tid < 256u) spare[c * 256u + tid] = 0u;
   const uint32_t n = *n_ptr;
   uint32_t t0, t1;
-  chunk_tiles(n, chunks, blockIdx.x, &t0, &t1);
+  chunk_tiles(n, chunks, c, &t0, &t1);
   if (t0 >= t1) return;
   if (tid < 2u) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.bar[tid])) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncthreads();
   uint32_t phases = 0;  // parity of the next phase of each buffer's barrier
   load_tile_bulk(keys_in, vals_in, t0 * kSortTile, n, s_buf, s_buf + kSortTile, smem_addr(&sm.bar[0]));
-  if (tid < RADIX) sm.run[tid] = offsets[(size_t)blockIdx.x * RADIX + tid];
-  for (uint32_t i = tid; i < kSortWarps * RADIX; i += kBlock) (&sm.warp_hist[0][0])[i] = 0u;
+  for (uint32_t i = tid; i < kSortWarps * RADIX * sizeof(uint16_t) / 4u; i += kScatterThreads)
+    reinterpret_cast<uint32_t*>(&sm.warp_hist[0][0])[i] = 0u;
+  // Thread d: the chunk's first position of digit d: keys of the digits below
+  // it, and of its own digit in the chunks before.
+  const uint32_t group = c / kSumChunks, groups = (chunks + kSumChunks - 1u) / kSumChunks;
+  uint32_t all = 0, before = 0;
+  if (tid < RADIX) {
+#pragma unroll 8
+    for (uint32_t g = 0; g < groups; ++g) {
+      const uint32_t x = sums[g * RADIX + tid];
+      all += x;
+      before += g < group ? x : 0u;
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < kSumChunks - 1u; ++r) {
+      const uint32_t row = group * kSumChunks + r;
+      before += row < c ? counts[(size_t)row * RADIX + tid] : 0u;
+    }
+  }
+  uint32_t run = digit_scan(all, sm.scan) + before;
 
   for (uint32_t t = t0; t < t1; ++t) {
     const uint32_t k = (t - t0) & 1u;
@@ -322,20 +357,19 @@ __global__ void __launch_bounds__(kBlock, kChunkBlocksPerSm)
     }
     const uint32_t base = t * kSortTile;
     if ((uint64_t)base + kSortTile <= n)
-      scatter_tile<BITS, true>(sm, kb, vb, base, n, shift, keys_out, vals_out);
+      scatter_tile<BITS, true>(sm, kb, vb, base, n, shift, keys_out, vals_out, run);
     else
-      scatter_tile<BITS, false>(sm, kb, vb, base, n, shift, keys_out, vals_out);
+      scatter_tile<BITS, false>(sm, kb, vb, base, n, shift, keys_out, vals_out, run);
   }
 }
 
 template <int B>
 void launch_chunk_bits(uint32_t chunks, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
-                       uint32_t* vals_out, const uint32_t* n_ptr, int shift, uint32_t* hist, uint32_t* counts,
-                       uint32_t* err, cudaStream_t st) {
-  k_chunk_count<B><<<chunks, kBlock, 0, st>>>(keys_in, n_ptr, shift, chunks, counts, hist);
-  k_chunk_offsets<B><<<1u << B, kBlock, 0, st>>>(hist, chunks, counts);
-  k_chunk_scatter<B><<<chunks, kBlock, kChunkDynSmem, st>>>(keys_in, vals_in, keys_out, vals_out, n_ptr, shift,
-                                                           chunks, counts, err);
+                       uint32_t* vals_out, const uint32_t* n_ptr, int shift, uint32_t* counts, uint32_t* sums,
+                       uint32_t* spare, uint32_t* err, cudaStream_t st) {
+  k_chunk_count<B><<<chunks, kBlock, 0, st>>>(keys_in, n_ptr, shift, chunks, counts, sums);
+  k_chunk_scatter<B><<<chunks, kScatterThreads, kChunkDynSmem, st>>>(keys_in, vals_in, keys_out, vals_out, n_ptr,
+                                                                    shift, chunks, counts, sums, spare, err);
 }
 
 template <int B>
@@ -354,11 +388,11 @@ uint32_t chunk_pass_chunks(uint32_t n_max, int sms) {
 }
 
 void launch_chunk_pass(int bits, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
-                       uint32_t* vals_out, const uint32_t* n_ptr, int shift, uint32_t* hist, uint32_t chunks,
-                       uint32_t* counts, uint32_t* err, cudaStream_t st) {
-#define GS_CHUNK(B)                                                                                             \
-  case B:                                                                                                       \
-    launch_chunk_bits<B>(chunks, keys_in, vals_in, keys_out, vals_out, n_ptr, shift, hist, counts, err, st);    \
+                       uint32_t* vals_out, const uint32_t* n_ptr, int shift, uint32_t chunks, uint32_t* counts,
+                       uint32_t* sums, uint32_t* spare, uint32_t* err, cudaStream_t st) {
+#define GS_CHUNK(B)                                                                                               \
+  case B:                                                                                                         \
+    launch_chunk_bits<B>(chunks, keys_in, vals_in, keys_out, vals_out, n_ptr, shift, counts, sums, spare, err, st); \
     break;
   switch (bits) {
     GS_CHUNK(1)
