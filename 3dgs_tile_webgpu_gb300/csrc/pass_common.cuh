@@ -264,7 +264,8 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
 // where (a, b, c) is the conic. Written by the projection when `rec` is not null.
 // rec: packed raster records of the fast forms (null for EXACT); erec: the
 // emission records, two float4 per item: (cx, cy, conic a, conic b),
-// (conic c, log(opacity * 255), rx + 512 ry, 0), written for visible items.
+// (conic c, log(opacity * 255), rx + 512 ry, 1 if the box has to be walked tile
+// by tile, else 0), written for visible items.
 void launch_project(const BatchView& b, const PassOptions& o, float4* mean, float4* conic, float4* color,
                     uint32_t* counts, uint32_t* keys, float4* rec, float4* erec, cudaStream_t st);
 // Starts a frame: advances the look-back epoch and clears `words` words (the

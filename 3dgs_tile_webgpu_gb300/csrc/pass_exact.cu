@@ -321,67 +321,45 @@ void launch_scan_counts(const uint32_t* ids, const uint32_t* tile_counts, uint32
 
 // ---------------------------------------------------------------------------
 // Emission kernel (emit_group, emission.cuh).
-// A block takes G groups of kBlock consecutive depth ranks and issues every
-// group's loads (ids, reserved counts, offsets, then the gathered mean and
-// conic) before working through the groups, so the gather latency of later
-// groups overlaps the earlier groups' work. Two groups pay off on large
-// launches (many blocks in flight anyway); one keeps small launches wide.
-constexpr uint32_t kEmitTwoGroupsFrom = 1u << 23;  // ranks per launch
-
-template <int G, bool PERIODIC>
-__global__ void __launch_bounds__(kBlock) k_emit(const uint32_t* __restrict__ ids, const float4* __restrict__ erec,
-                                                 const uint32_t* __restrict__ ordered,
-                                                 const uint32_t* __restrict__ offsets, BatchView bv, PassOptions o,
-                                                 Control* __restrict__ ctl, uint32_t capacity,
-                                                 uint32_t* __restrict__ tile_keys, uint32_t* __restrict__ tile_vals) {
+// A block takes kBlock consecutive depth ranks. 5 blocks per SM (48
+// registers): with no bound (60 registers, 4 blocks) 6M ranks took 206 us
+// instead of 193, and two groups of ranks per block (64 registers; it paid
+// off while the box rows were walked tile by tile) 1153 us instead of 1113 for
+// 2 x 17.5M ranks.
+template <bool PERIODIC>
+__global__ void __launch_bounds__(kBlock, 5) k_emit(const uint32_t* __restrict__ ids, const float4* __restrict__ erec,
+                                                    const uint32_t* __restrict__ ordered,
+                                                    const uint32_t* __restrict__ offsets, BatchView bv, PassOptions o,
+                                                    Control* __restrict__ ctl, uint32_t capacity,
+                                                    uint32_t* __restrict__ tile_keys,
+                                                    uint32_t* __restrict__ tile_vals) {
   if (ctl->state[3] != 0u) return;  // overflow: emission dispatch is zero
   __shared__ EmitShared sm;
-  const uint32_t tid = threadIdx.x;
   const uint32_t n = ctl->visible_state[0];
-  const uint32_t first = blockIdx.x * kBlock * G;
+  const uint32_t first = blockIdx.x * kBlock;
   if (first >= n) return;  // whole block past the visible count
-  uint32_t g[G], res[G], off[G];
-  float4 e0[G], e1[G];
-#pragma unroll
-  for (int h = 0; h < G; ++h) {
-    const uint32_t r = first + (uint32_t)h * kBlock + tid;
-    g[h] = 0u; res[h] = 0u; off[h] = 0u;
-    if (r < n) {
-      g[h] = ids[r];
-      res[h] = ordered[r];
-      off[h] = offsets[r];
-    }
+  const uint32_t r = first + threadIdx.x;
+  uint32_t g = 0u, reserved = 0u, offset = 0u;
+  float4 e0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), e1 = e0;
+  if (r < n) {
+    g = ids[r];
+    reserved = ordered[r];
+    offset = offsets[r];
+    e0 = __ldg(erec + 2 * (size_t)g);
+    e1 = __ldg(erec + 2 * (size_t)g + 1);
   }
-#pragma unroll
-  for (int h = 0; h < G; ++h) {
-    const uint32_t r = first + (uint32_t)h * kBlock + tid;
-    e0[h] = e1[h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (r < n) {
-      e0[h] = __ldg(erec + 2 * (size_t)g[h]);
-      e1[h] = __ldg(erec + 2 * (size_t)g[h] + 1);
-    }
-  }
-#pragma unroll
-  for (int h = 0; h < G; ++h) {
-    const uint32_t r = first + (uint32_t)h * kBlock + tid;
-    emit_group<PERIODIC>(sm, r < n, g[h], e0[h], e1[h], res[h], off[h], bv, o, capacity, tile_keys, tile_vals);
-  }
+  emit_group<PERIODIC>(sm, r < n, g, e0, e1, reserved, offset, bv, o, capacity, tile_keys, tile_vals);
 }
 
 void launch_emit(const uint32_t* ids, uint32_t n_max, const float4* erec, const uint32_t* ordered,
                  const uint32_t* offsets, const BatchView& b, const PassOptions& o, Control* ctl, uint32_t capacity,
                  uint32_t* tile_keys, uint32_t* tile_vals, cudaStream_t st) {
   if (n_max == 0) return;
-  const uint32_t per = n_max >= kEmitTwoGroupsFrom ? 2u * kBlock : kBlock;
-  const uint32_t grid = (n_max - 1u) / per + 1u;
-#define GS_EMIT(G, P) \
-  k_emit<G, P><<<grid, kBlock, 0, st>>>(ids, erec, ordered, offsets, b, o, ctl, capacity, tile_keys, tile_vals)
-  if (per == kBlock) {
-    if (o.axis) GS_EMIT(1, true); else GS_EMIT(1, false);
-  } else {
-    if (o.axis) GS_EMIT(2, true); else GS_EMIT(2, false);
-  }
-#undef GS_EMIT
+  const uint32_t grid = (n_max - 1u) / kBlock + 1u;
+  if (o.axis)
+    k_emit<true><<<grid, kBlock, 0, st>>>(ids, erec, ordered, offsets, b, o, ctl, capacity, tile_keys, tile_vals);
+  else
+    k_emit<false><<<grid, kBlock, 0, st>>>(ids, erec, ordered, offsets, b, o, ctl, capacity, tile_keys, tile_vals);
 }
 
 // ---------------------------------------------------------------------------

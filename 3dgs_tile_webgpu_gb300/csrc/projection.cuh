@@ -63,9 +63,10 @@ __device__ __forceinline__ uint32_t bit_range(uint32_t s, uint32_t e) {
   return (e >= 32u ? 0xffffffffu : ((1u << e) - 1u)) & ~((1u << s) - 1u);
 }
 
-// Boxes of at least this many tiles are walked by the whole warp, one box at
-// a time, instead of in the shared rounds of the tile count and the emission:
-// no per-tile owner lookup, the owner's parameters broadcast to every lane.
+// Boxes along a periodic axis of at least this many tiles are walked by the
+// whole warp, one box at a time, instead of in the shared rounds of the tile
+// count and the emission: no per-tile owner lookup, the owner's parameters
+// broadcast to every lane.
 constexpr uint32_t kWideBox = 64;
 
 // The tiles a splat may reach, walked in row-major order: bw columns and bh
@@ -145,6 +146,106 @@ __device__ __forceinline__ TileBox tile_box(float cx, float cy, float rx, float 
   return t;
 }
 
+// Boxes of at least this many tiles are counted and emitted row by row
+// (row_span): a lane finds the tiles of one box row that pass the reference's
+// tile test without testing each. Projection and emission, us, with all boxes
+// walked tile by tile and with rows from 96 / 64 / 32 / 12 tiles on: 12M
+// splats at 4K (398M records) 4074 + 3767, and 2814 + 2344, 2668 + 2245,
+// 2486 + 2105, 2384 + 1948; 16 views of 3M splats (85M records, mostly small
+// boxes) 2877 + 1106, and 2849 + 1198, 2849 + 1198, 2863 + 1202, 3236 + 1270
+// (an emission kernel since replaced: 1737 and 1098 from 32 on).
+constexpr uint32_t kRowBox = 32;
+
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float y;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// The tiles of one box row that pass tile_rect_test, [first, last] (empty:
+// last < first). Not `regular`: the row's hits are not one run, or the conic is
+// too near singular to bound the test's rounding; the box is then walked tile
+// by tile.
+struct RowSpan {
+  int first, last;
+  bool regular;
+};
+
+// The splat's support {q(d) <= 2 thr}, cut by the row's y range, projects onto an
+// interval of x; a tile passes when it meets the interval. The ends follow
+// from the conic: the support's rightmost point lies at dy = -(k1 / k2) X with
+// X = sqrt(2 thr k2 / det), its boundary at dy is
+// x = (-k1 dy +- sqrt(2 thr k0 - det dy^2)) / k0, and the end over the row is
+// the boundary at that dy clamped to the row. The interval is taken once with
+// the threshold raised by `delta` and the row and the ends widened by `m`
+// pixels, once with both the other way: tiles outside the wide one fail, tiles
+// that meet the narrow one pass, and those between (mostly none) are tested as
+// the reference does. delta and m bound the rounding of the reference's test:
+// its sigma is off by at most a few 2^-24 times k0 dx^2 + k2 dy^2 + 2 |k1 dx dy|,
+// which at the boundary is below 4 k0 k2 / det thr, and its dx, dy by a
+// few units in the last place of the coordinates.
+__device__ __forceinline__ RowSpan row_span(float cx, float cy, float k0, float k1, float k2, float thr, int ty,
+                                            int x0, int x1, float extent, float ts, float inv) {
+  RowSpan s = {1, 0, true};
+  const float p = k1 * k1;
+  const float det = __fmaf_rn(k0, k2, -p) - __fmaf_rn(k1, k1, -p);  // k0 k2 - k1^2 without its cancellation error
+  const float delta = 1e-3f + 4e-6f * __fdividef(k0 * k2, det);
+  if (!(k0 > 0.0f && k2 > 0.0f && det > 0.0f && delta < 0.25f)) {
+    s.regular = false;
+    return s;
+  }
+  const float m = 0.02f + 1e-6f * (fabsf(cx) + fabsf(cy) + extent);
+  const float ik0 = __fdividef(1.0f, k0), slope = __fdividef(k1, k2), x2 = __fdividef(k2, det);
+  const float y0 = (float)ty * ts - cy, y1 = y0 + ts;
+  int a0 = 0, b0 = -1, a1 = 0, b1 = -1;
+#pragma unroll
+  for (int wide = 1; wide >= 0; --wide) {
+    const float grow = wide ? m : -m;
+    const float level = (2.0f * thr) * (wide ? 1.0f + delta : 1.0f - delta);
+    const float lo = y0 - grow, hi = y1 + grow, top = k0 * level;
+    const float nearest = fminf(fmaxf(0.0f, lo), hi);
+    if (!(top >= det * nearest * nearest)) break;  // the row misses the support
+    const float yr = slope * sqrt_approx(level * x2);
+    const float dr = fminf(fmaxf(-yr, lo), hi), dl = fminf(fmaxf(yr, lo), hi);
+    const float xr = cx + (sqrt_approx(fmaxf(top - det * dr * dr, 0.0f)) - k1 * dr) * ik0 + grow;
+    const float xl = cx - (sqrt_approx(fmaxf(top - det * dl * dl, 0.0f)) + k1 * dl) * ik0 - grow;
+    if (wide) {
+      a0 = max((int)floorf(xl * inv), x0);
+      b0 = min((int)floorf(xr * inv), x1);
+    } else if (xl <= xr) {
+      a1 = max((int)floorf(xl * inv), a0);
+      b1 = min((int)floorf(xr * inv), b0);
+    }
+  }
+  if (a0 > b0) return s;
+  const bool core = a1 <= b1;
+  int hits = core ? b1 - a1 + 1 : 0;
+  if (b0 - a0 + 1 - hits > 8) {
+    s.regular = false;
+    return s;
+  }
+  s.first = core ? a1 : b0 + 1;
+  s.last = core ? b1 : a0 - 1;
+  for (int t = a0; t <= b0; ++t) {
+    if (core && t == a1) {
+      t = b1;
+      continue;
+    }
+    if (tile_rect_test(cx, cy, k0, k1, k2, thr, t, ty, ts)) {
+      s.first = min(s.first, t);
+      s.last = max(s.last, t);
+      ++hits;
+    }
+  }
+  if (hits == 0) {
+    s.first = 1;
+    s.last = 0;
+  } else {
+    s.regular = s.last - s.first + 1 == hits;
+  }
+  return s;
+}
+
 // Per-warp tables of the projection's cooperative tile count: the splat
 // parameters of the tile test, the box, and the inclusive box-tile counts.
 struct CountShared {
@@ -154,27 +255,43 @@ struct CountShared {
   uint32_t cnt[kBlock / 32][32];
 };
 
-// Counts the tiles of every lane's box that pass the reference's tile test,
-// with the warp's lanes spread over the union of the 32 boxes (32 box tiles
-// per round) instead of each lane walking its own box. A lane walks nbox
-// tiles of its box in row-major order, skipping the box index u[3] (the
-// centre's tile, counted by the caller); boxes of kWideBox tiles or more are
-// walked afterwards by the whole warp, one at a time. Must be called by all
-// 32 lanes; a lane with nbox == 0 contributes nothing. Returns the lane's
-// count.
-template <bool PERIODIC>
-__device__ __forceinline__ uint32_t count_tiles_warp(CountShared& sm, uint32_t nbox, float vw, float vh,
-                                                     uint32_t axis, float ts) {
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  // Wide boxes (kWideBox tiles or more) are left out of the shared rounds and
-  // walked by the whole warp afterwards, one box at a time.
-  const bool wide = nbox >= kWideBox;
-  uint32_t incl = wide ? 0u : nbox;
+// The lane whose run of an inclusive scan holds j (the scan's total is above j).
+__device__ __forceinline__ uint32_t find_owner(const uint32_t* incl, uint32_t j) {
+  uint32_t owner = 0;
+#pragma unroll
+  for (uint32_t step = 16; step >= 1; step >>= 1)
+    if (incl[owner + step - 1] <= j) owner += step;
+  return owner;
+}
+
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v) {
+  const uint32_t lane = threadIdx.x & 31u;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= (uint32_t)d) incl += y;
+    const uint32_t y = __shfl_up_sync(0xffffffffu, v, d);
+    if (lane >= (uint32_t)d) v += y;
   }
+  return v;
+}
+
+// Counts the tiles of every lane's box (nbox tiles in rows rows) that pass the
+// reference's tile test, with the warp's lanes spread over the union of the
+// 32 boxes instead of each lane walking its own. Small boxes share
+// rounds of 32 tiles, in row-major order; the centre's tile (`centre`, box
+// index u[3]) counts without a test. Boxes of kRowBox tiles or more share rounds
+// of 32 rows. Boxes those cannot take (*irregular), and wide ones along a
+// periodic axis, are walked tile by tile by the whole warp, one at a time.
+// Must be called by all 32 lanes; a lane with nbox == 0 contributes nothing.
+// Returns the lane's count.
+template <bool PERIODIC>
+__device__ __forceinline__ uint32_t count_tiles_warp(CountShared& sm, uint32_t nbox, uint32_t rows, bool centre,
+                                                     float vw, float vh, uint32_t axis, float ts, float inv,
+                                                     bool* irregular) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const bool by_rows = !PERIODIC && nbox >= kRowBox;
+  bool wide = PERIODIC && nbox >= kWideBox;
+  const uint32_t walk = centre ? nbox - 1u : nbox;  // the tile walks skip the centre's tile
+  const uint32_t incl = warp_inclusive(wide || by_rows ? 0u : walk);
   sm.incl[warp][lane] = incl;
   sm.cnt[warp][lane] = 0u;
   __syncwarp();
@@ -182,10 +299,7 @@ __device__ __forceinline__ uint32_t count_tiles_warp(CountShared& sm, uint32_t n
   for (uint32_t j0 = 0; j0 < total; j0 += 32) {
     const uint32_t j = j0 + lane;
     const bool valid = j < total;
-    uint32_t owner = 0;
-#pragma unroll
-    for (uint32_t step = 16; step >= 1; step >>= 1)
-      if (sm.incl[warp][owner + step - 1] <= j) owner += step;
+    const uint32_t owner = find_owner(sm.incl[warp], j);
     bool hit = false;
     if (valid) {
       const uint32_t bw = sm.u[2][warp][owner];
@@ -203,8 +317,37 @@ __device__ __forceinline__ uint32_t count_tiles_warp(CountShared& sm, uint32_t n
     if (valid && lane == 31u - (uint32_t)__clz(same)) sm.cnt[warp][owner] += __popc(hits & same);
   }
   __syncwarp();
-  uint32_t cnt = sm.cnt[warp][lane];
-  // Wide boxes: the whole warp walks one box, 32 tiles a step.
+  uint32_t cnt = sm.cnt[warp][lane] + (centre && !by_rows ? 1u : 0u);
+  if (!PERIODIC && __any_sync(0xffffffffu, by_rows)) {
+    // Rounds of 32 box rows.
+    const uint32_t rincl = warp_inclusive(by_rows ? rows : 0u);
+    sm.incl[warp][lane] = rincl;
+    sm.cnt[warp][lane] = 0u;
+    __syncwarp();
+    const uint32_t rtotal = __shfl_sync(0xffffffffu, rincl, 31);
+    for (uint32_t j0 = 0; j0 < rtotal; j0 += 32) {
+      const uint32_t j = j0 + lane;
+      if (j < rtotal) {
+        const uint32_t owner = find_owner(sm.incl[warp], j);
+        const uint32_t row = j - (owner ? sm.incl[warp][owner - 1] : 0u);
+        const int x0 = (int)sm.u[0][warp][owner];
+        const RowSpan r = row_span(sm.f[0][warp][owner], sm.f[1][warp][owner], sm.f[2][warp][owner],
+                                   sm.f[3][warp][owner], sm.f[4][warp][owner], sm.f[5][warp][owner],
+                                   (int)(sm.u[1][warp][owner] + row), x0, x0 + (int)sm.u[2][warp][owner] - 1, vw + vh,
+                                   ts, inv);
+        // The sign bit marks a box that needs the tile walk.
+        if (!r.regular) atomicOr(&sm.cnt[warp][owner], 0x80000000u);
+        else if (r.last >= r.first) atomicAdd(&sm.cnt[warp][owner], (uint32_t)(r.last - r.first + 1));
+      }
+    }
+    __syncwarp();
+    if (by_rows) {
+      cnt = sm.cnt[warp][lane];
+      wide = (cnt >> 31) != 0u;
+    }
+  }
+  *irregular = wide;
+  // The whole warp walks one box, 32 tiles a step.
   uint32_t wide_lanes = __ballot_sync(0xffffffffu, wide);
   while (wide_lanes) {
     const uint32_t w = (uint32_t)__ffs(wide_lanes) - 1u;
@@ -213,7 +356,7 @@ __device__ __forceinline__ uint32_t count_tiles_warp(CountShared& sm, uint32_t n
     // (broadcast loads) rather than held in registers across the walk.
     const volatile float(*vf)[kBlock / 32][32] = sm.f;
     const volatile uint32_t(*vu)[kBlock / 32][32] = sm.u;
-    const uint32_t n = __shfl_sync(0xffffffffu, nbox, w);
+    const uint32_t n = __shfl_sync(0xffffffffu, walk, w);
     uint32_t sum = 0;
     for (uint32_t j0 = 0; j0 < n; j0 += 32) {
       uint32_t k = j0 + lane;
@@ -229,7 +372,7 @@ __device__ __forceinline__ uint32_t count_tiles_warp(CountShared& sm, uint32_t n
       }
       sum += __popc(__ballot_sync(0xffffffffu, hit));
     }
-    if (lane == w) cnt = sum;
+    if (lane == w) cnt = sum + (centre ? 1u : 0u);
   }
   return cnt;
 }
@@ -285,8 +428,8 @@ __device__ __forceinline__ void project_block(uint32_t block, const BatchView& b
     const uint32_t item = v.item_base + gid;
     const float vw = v.vw, vh = v.vh;
     float4 mo4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    uint32_t cnt = 0, key = kInvisibleKey, nbox = 0;
-    bool centre = false;
+    uint32_t cnt = 0, key = kInvisibleKey, nbox = 0, rows = 0;
+    bool centre = false, irregular = false;
     Projected pr = {};
     float op = 0.0f, rx = 0.0f, ry = 0.0f, thr = 0.0f;
     float ddx = 0.0f, ddy = 0.0f, ddz = 0.0f;  // positionLocal - cameraLocal
@@ -362,6 +505,7 @@ __device__ __forceinline__ void project_block(uint32_t block, const BatchView& b
       const TileBox box = tile_box<PERIODIC>(pr.cx, pr.cy, rx, ry, vw, vh, (int)v.tiles_x, (int)v.tiles_y, o);
       const float mtx = (float)((int)v.tiles_x - 1), mty = (float)((int)v.tiles_y - 1);
       nbox = box.bw * box.bh;
+      rows = box.bh;
       // The tile holding the centre, when it is on screen, lies in the box
       // (the floors are monotone and rx, ry >= 1) and passes the reference's
       // tile test by its centre-inside path (tileContribution.ts:16-59): it
@@ -379,7 +523,7 @@ __device__ __forceinline__ void project_block(uint32_t block, const BatchView& b
       if (PERIODIC) s_count.u[4][warp][lane] = box.wrap;
     } while (false);
     // Tiles passing the tile test (projectionHelpers.ts:223-236), counted by the whole warp.
-    cnt = count_tiles_warp<PERIODIC>(s_count, centre ? nbox - 1u : nbox, vw, vh, o.axis, o.tile_px) + (centre ? 1u : 0u);
+    cnt = count_tiles_warp<PERIODIC>(s_count, nbox, rows, centre, vw, vh, o.axis, o.tile_px, o.tile_inv, &irregular);
     if (cnt > 0) {
       uint32_t co[16];
       load_sh(v.sh + (size_t)slot * v.C, v.degree, co);
@@ -401,7 +545,7 @@ __device__ __forceinline__ void project_block(uint32_t block, const BatchView& b
       // Emission record: what the emission reads per depth rank, in one
       // 32-byte gather (layout in pass_common.cuh).
       erec_out[2 * (size_t)item] = make_float4(pr.cx, pr.cy, pr.conic_x, pr.conic_y);
-      erec_out[2 * (size_t)item + 1] = make_float4(pr.conic_z, thr, rx + ry * 512.0f, 0.0f);
+      erec_out[2 * (size_t)item + 1] = make_float4(pr.conic_z, thr, rx + ry * 512.0f, irregular ? 1.0f : 0.0f);
       color_out[item] = make_float4(col.x, col.y, col.z, __uint_as_float(slot ^ kActiveTag));
       if (rec_out) {
         // Packed raster record of the fast forms (layout in pass_common.cuh).
