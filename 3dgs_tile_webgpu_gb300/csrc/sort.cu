@@ -22,23 +22,27 @@
 //                   own in its group (at most 29 + 15 rows; a kernel between
 //                   the two that turned the counts into positions took 6 us a
 //                   pass), then walks its tiles in order with running
-//                   per-digit offsets: tile t+1 streams into shared memory by
-//                   two bulk copies (cp.async.bulk, 16 KB of keys and 16 KB
-//                   of values, completion counted on an mbarrier) while tile
-//                   t is ranked per digit within each warp by ballot
-//                   bit-splitting (warp-striped layout: item j*32+lane of
+//                   per-digit offsets: the keys of tile t+1 stream into
+//                   shared memory by a bulk copy (cp.async.bulk, completion
+//                   counted on an mbarrier) while tile t is ranked per digit
+//                   within each warp (warp-striped layout: item j*32+lane of
 //                   each warp's 512-item segment, so ranks follow index
 //                   order), staged in place in block-sorted order, and
-//                   written out with each digit's run contiguous.
+//                   written out with each digit's run contiguous; its values
+//                   stream in while it is ranked.
 // Stable: tiles in index order within a chunk, chunks in index order, ranks in
 // index order within a tile.
-// Bound by instructions and shared memory (ballots, one look-up and two random
-// stores per item), not by HBM. us, with offsets kernel, equal chunk sizes and
-// two look-ups -> so: depth sort of 2.3M / 6M / 2 x 17.5M items 156 -> 122,
-// 253 -> 208, 1125 -> 1087; tile sort of 5.5M / 17.7M / 2 x 42.7M / 398M
-// records 97 -> 83, 252 -> 229, 1252 -> 1199, 5433 -> 5286 (2.4 TB/s of
-// scattered writes and reads). 512 threads of 8 items spill at 40 registers:
-// 1201 and 1323 for the 16 views.
+// Bound by instructions and shared memory, not by HBM (2.4 TB/s at 398M
+// records). The lanes of a digit are found by 8 ballots (95 instructions and 21
+// shared-memory wavefronts per 32 items in all) or by each lane setting its bit
+// in its digit's word (60 and 32): ballots alone keep the issue slots busy, the
+// words alone the shared memory (73% of its wavefronts), so the rows of a
+// warp take turns. us, depth sort of 6M items / of 2 x 17.5M, tile sort of
+// 17.7M / 398M records: ballots 213 / 1099 / 230 / 5418, words 191 / 1083 / 211 /
+// 5151, turns 191 / 1057 / 206 / 5028. Three of four rows by ballots 205 / 1080 /
+// 218 / 5233. The tables leave no room for two value buffers; single buffers
+// and 4 blocks per SM: 203 / 1119 / 224 / 5523; 512 threads of 8 items spill at 40
+// registers (1201 for 2 x 17.5M).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -128,16 +132,17 @@ __global__ void __launch_bounds__(kBlock) k_chunk_count(const uint32_t* __restri
   }
 }
 
-// Two tile buffers (keys and values each): tile t+1 streams in while tile t
-// is ranked and scattered.
-constexpr size_t kChunkDynSmem = 2 * 2 * kSortTile * sizeof(uint32_t);
+// Two buffers of keys, one of values: the keys of tile t+1 stream in while
+// tile t is ranked and scattered, its values while it is ranked.
+constexpr size_t kChunkDynSmem = 3 * kSortTile * sizeof(uint32_t);
 
 template <int BITS>
 struct ScatterShared {
   uint16_t warp_hist[kSortWarps][1u << BITS];  // a warp's items per digit, then its first tile position
+  uint32_t match[kSortWarps][1u << BITS];  // lanes of the warp's current row holding each digit; zero in between
   uint32_t delta[1u << BITS];  // global position of the tile's item i of a digit, minus i
   uint32_t scan[8];
-  unsigned long long bar[2];  // bulk-copy completion of each tile buffer
+  unsigned long long bar[3];  // bulk-copy completion of the two key buffers and the value buffer
 };
 
 // Exclusive scan of one value per digit over the threads below 256, in two
@@ -160,34 +165,26 @@ __device__ __forceinline__ uint32_t digit_scan(uint32_t v, uint32_t* s_scan) {
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// Bulk copies of one tile's keys and values (items base .. min(base + 4096,
-// n)) into kb/vb, issued by thread 0 and counted on the buffer's mbarrier;
-// the last n % 4 items of a ragged tile (a bulk copy moves whole 16-byte
-// units) come by plain loads, visible after the next block barrier.
-__device__ __forceinline__ void load_tile_bulk(const uint32_t* __restrict__ keys_in,
-                                               const uint32_t* __restrict__ vals_in, uint32_t base, uint32_t n,
-                                               uint32_t* kb, uint32_t* vb, uint32_t bar) {
+// Bulk copy of one tile's keys or values (items base .. min(base + 4096, n))
+// into buf, issued by thread 0 and counted on the mbarrier; the last n % 4
+// items of a ragged tile (a bulk copy moves whole 16-byte units) come by plain
+// loads, visible after the next block barrier.
+__device__ __forceinline__ void load_tile_bulk(const uint32_t* __restrict__ in, uint32_t base, uint32_t n,
+                                               uint32_t* buf, uint32_t bar) {
   const uint32_t items = min(kSortTile, n - base);
-  const uint32_t whole = items & ~3u;  // items moved by the bulk copies
+  const uint32_t whole = items & ~3u;  // items moved by the bulk copy
   if (threadIdx.x == 0) {
     const uint32_t bytes = whole * 4u;
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2u * bytes) : "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
     if (bytes) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the buffer's previous reads come first
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                       smem_addr(kb)),
-                   "l"(keys_in + base), "r"(bytes), "r"(bar)
-                   : "memory");
-      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                       smem_addr(vb)),
-                   "l"(vals_in + base), "r"(bytes), "r"(bar)
+                       smem_addr(buf)),
+                   "l"(in + base), "r"(bytes), "r"(bar)
                    : "memory");
     }
   }
-  for (uint32_t e = whole + threadIdx.x; e < items; e += kScatterThreads) {
-    kb[e] = keys_in[base + e];
-    vb[e] = vals_in[base + e];
-  }
+  for (uint32_t e = whole + threadIdx.x; e < items; e += kScatterThreads) buf[e] = in[base + e];
 }
 
 // Bounded wait for phase `parity` of the mbarrier (about a second of polls).
@@ -211,11 +208,12 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
 // stages it in place in block-sorted order and writes each digit's run to its
 // global position. FULL: every item of the tile is below n. `run`: the global
 // position of the next item of digit threadIdx.x (threads below 2^BITS).
-// Leaves warp_hist zeroed and run advanced past the tile.
+// Leaves warp_hist zeroed and run advanced past the tile. parity: the phase of
+// the value buffer's barrier; false if the values never landed.
 template <int BITS, bool FULL>
-__device__ __forceinline__ void scatter_tile(ScatterShared<BITS>& sm, uint32_t* kb, uint32_t* vb, uint32_t base,
+__device__ __forceinline__ bool scatter_tile(ScatterShared<BITS>& sm, uint32_t* kb, uint32_t* vb, uint32_t base,
                                              uint32_t n, int shift, uint32_t* __restrict__ keys_out,
-                                             uint32_t* __restrict__ vals_out, uint32_t& run) {
+                                             uint32_t* __restrict__ vals_out, uint32_t& run, uint32_t parity) {
   constexpr uint32_t RADIX = 1u << BITS;
   constexpr uint32_t MASK = RADIX - 1u;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -229,13 +227,25 @@ __device__ __forceinline__ void scatter_tile(ScatterShared<BITS>& sm, uint32_t* 
     const bool ok = FULL || base + wofs + (uint32_t)j * 32u + lane < n;
     const uint32_t valid = FULL ? 0xffffffffu : __ballot_sync(0xffffffffu, ok);
     const uint32_t d = (k[j] >> shift) & MASK;
-    const uint32_t peers = match_digit<BITS>(d, valid);
+    uint32_t peers = valid;
+    if (!FULL || (j & 1)) {
+      peers = match_digit<BITS>(d, valid);
+    } else if (!__all_sync(0xffffffffu, d == __shfl_sync(0xffffffffu, d, 0))) {
+      // Each lane sets its bit in its digit's word; one digit for the whole
+      // row would serialise the 32 atomics and needs none.
+      atomicOr(&sm.match[warp][d], 1u << lane);
+      __syncwarp();
+      peers = sm.match[warp][d];
+    }
     const uint32_t before = __popc(peers & lt);
     uint32_t cnt = 0;
     if (ok) cnt = sm.warp_hist[warp][d];
     rank[j] = cnt + before;
     __syncwarp();
-    if (ok && before == 0) sm.warp_hist[warp][d] = (uint16_t)(cnt + __popc(peers));
+    if (ok && before == 0) {
+      sm.warp_hist[warp][d] = (uint16_t)(cnt + __popc(peers));
+      if (FULL && !(j & 1)) sm.match[warp][d] = 0u;
+    }
     __syncwarp();
   }
   __syncthreads();
@@ -272,9 +282,10 @@ __device__ __forceinline__ void scatter_tile(ScatterShared<BITS>& sm, uint32_t* 
       kb[rank[j]] = k[j];
     }
   }
+  const bool landed = bar_wait(smem_addr(&sm.bar[2]), parity);
 #pragma unroll
   for (int j = 0; j < kSortItems; ++j) k[j] = vb[wofs + (uint32_t)j * 32u + lane];
-  __syncthreads();
+  if (!__syncthreads_and(landed)) return false;
 #pragma unroll
   for (int j = 0; j < kSortItems; ++j)
     if (FULL || base + wofs + (uint32_t)j * 32u + lane < n) vb[rank[j]] = k[j];
@@ -291,6 +302,7 @@ __device__ __forceinline__ void scatter_tile(ScatterShared<BITS>& sm, uint32_t* 
   for (uint32_t i = tid; i < kSortWarps * RADIX * sizeof(uint16_t) / 4u; i += kScatterThreads)
     reinterpret_cast<uint32_t*>(&sm.warp_hist[0][0])[i] = 0u;
   __syncthreads();
+  return true;
 }
 
 template <int BITS>
@@ -312,11 +324,13 @@ __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
   uint32_t t0, t1;
   chunk_tiles(n, chunks, c, &t0, &t1);
   if (t0 >= t1) return;
-  if (tid < 2u) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.bar[tid])) : "memory");
+  if (tid < 3u) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.bar[tid])) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncthreads();
   uint32_t phases = 0;  // parity of the next phase of each buffer's barrier
-  load_tile_bulk(keys_in, vals_in, t0 * kSortTile, n, s_buf, s_buf + kSortTile, smem_addr(&sm.bar[0]));
+  uint32_t* vb = s_buf + 2u * kSortTile;
+  load_tile_bulk(keys_in, t0 * kSortTile, n, s_buf, smem_addr(&sm.bar[0]));
+  for (uint32_t i = tid; i < kSortWarps * RADIX; i += kScatterThreads) (&sm.match[0][0])[i] = 0u;
   for (uint32_t i = tid; i < kSortWarps * RADIX * sizeof(uint16_t) / 4u; i += kScatterThreads)
     reinterpret_cast<uint32_t*>(&sm.warp_hist[0][0])[i] = 0u;
   // Thread d: the chunk's first position of digit d: keys of the digits below
@@ -339,27 +353,29 @@ __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
   uint32_t run = digit_scan(all, sm.scan) + before;
 
   for (uint32_t t = t0; t < t1; ++t) {
-    const uint32_t k = (t - t0) & 1u;
-    uint32_t* kb = s_buf + k * 2u * kSortTile;
-    uint32_t* vb = kb + kSortTile;
-    if (t + 1u < t1) {
-      uint32_t* nb = s_buf + (k ^ 1u) * 2u * kSortTile;
-      load_tile_bulk(keys_in, vals_in, (t + 1u) * kSortTile, n, nb, nb + kSortTile, smem_addr(&sm.bar[k ^ 1u]));
+    const uint32_t k = (t - t0) & 1u, base = t * kSortTile;
+    uint32_t* kb = s_buf + k * kSortTile;
+    load_tile_bulk(vals_in, base, n, vb, smem_addr(&sm.bar[2]));
+    if (t + 1u < t1)
+      load_tile_bulk(keys_in, base + kSortTile, n, s_buf + (k ^ 1u) * kSortTile, smem_addr(&sm.bar[k ^ 1u]));
+    bool ok = __syncthreads_and(bar_wait(smem_addr(&sm.bar[k]), (phases >> k) & 1u));
+    const uint32_t parity = (t - t0) & 1u;
+    if (ok) {
+      if ((uint64_t)base + kSortTile <= n)
+        ok = scatter_tile<BITS, true>(sm, kb, vb, base, n, shift, keys_out, vals_out, run, parity);
+      else
+        ok = scatter_tile<BITS, false>(sm, kb, vb, base, n, shift, keys_out, vals_out, run, parity);
+    } else {
+      bar_wait(smem_addr(&sm.bar[2]), parity);
     }
-    const bool landed = bar_wait(smem_addr(&sm.bar[k]), (phases >> k) & 1u);
     phases ^= 1u << k;
-    if (!__syncthreads_and(landed)) {
-      // A copy never landed: flag the frame and leave, after the other
-      // buffer's copy (if one was issued) had its own bounded wait.
+    if (!ok) {
+      // A copy never landed: flag the frame and leave, after the copy of the
+      // next keys (if one was issued) had its own bounded wait.
       if (tid == 0) atomicOr(err, 4u);
       if (t + 1u < t1) bar_wait(smem_addr(&sm.bar[k ^ 1u]), (phases >> (k ^ 1u)) & 1u);
       return;
     }
-    const uint32_t base = t * kSortTile;
-    if ((uint64_t)base + kSortTile <= n)
-      scatter_tile<BITS, true>(sm, kb, vb, base, n, shift, keys_out, vals_out, run);
-    else
-      scatter_tile<BITS, false>(sm, kb, vb, base, n, shift, keys_out, vals_out, run);
   }
 }
 
