@@ -454,9 +454,13 @@ __device__ __forceinline__ void project_block(uint32_t block, const BatchView& b
       double vxd = 0.0, vyd = 0.0, vzd = 0.0;
       float vx, vy, vz;
       if (FP64) {
-        vxd = (((double)mv[0] * mo.x + (double)mv[4] * mo.y) + (double)mv[8] * mo.z) + (double)mv[12];
-        vyd = (((double)mv[1] * mo.x + (double)mv[5] * mo.y) + (double)mv[9] * mo.z) + (double)mv[13];
-        vzd = (((double)mv[2] * mo.x + (double)mv[6] * mo.y) + (double)mv[10] * mo.z) + (double)mv[14];
+        // A product of two floats is exact in double, so a fused multiply-add
+        // rounds like the product and the sum; the FP64 unit (2 lanes per SM)
+        // is what this form waits for.
+        const double px = mo.x, py = mo.y, pz = mo.z;
+        vxd = __fma_rn((double)mv[8], pz, __fma_rn((double)mv[4], py, (double)mv[0] * px)) + (double)mv[12];
+        vyd = __fma_rn((double)mv[9], pz, __fma_rn((double)mv[5], py, (double)mv[1] * px)) + (double)mv[13];
+        vzd = __fma_rn((double)mv[10], pz, __fma_rn((double)mv[6], py, (double)mv[2] * px)) + (double)mv[14];
         vx = (float)vxd; vy = (float)vyd; vz = (float)vzd;
       } else {
         vx = ((mv[0] * mo.x + mv[4] * mo.y) + mv[8] * mo.z) + mv[12] * 1.0f;
