@@ -287,20 +287,22 @@ void launch_emit(const uint32_t* sorted_ids, uint32_t n_max, const float4* erec,
 void launch_tile_ranges(const uint32_t* sorted_tile_keys, Control* ctl, uint32_t ntile, uint32_t n_max,
                         uint32_t* tile_offsets, cudaStream_t st);
 constexpr uint32_t kSortTile = 4096;  // items per sort tile
-// Chunked LSD pass (reduce, scatter; no look-back chain): `chunks` blocks,
-// each walking a contiguous run of 4096-item tiles. counts holds chunks rows
-// of 2^bits words; sums (sum_rows(chunks) rows of 256 words, zero on entry)
-// takes the counts of 16 chunks a row; spare, as large, is zeroed (the next
-// pass takes it as its sums). n is read from *n_ptr on the device.
+// Chunked LSD pass (reduce, scatter; no look-back chain) over the digit of
+// `bits` bits from `shift` on of the key, or, at 9 bits (the most), of
+// key - low: `chunks` blocks, each walking a contiguous run of 4096-item tiles. counts holds chunks rows
+// of 2^bits words; sums (sum_rows(chunks) rows of kSumWords words, zero on
+// entry) takes the counts of 16 chunks a row; spare, as large, is zeroed (the
+// next pass takes it as its sums). n is read from *n_ptr on the device.
 constexpr uint32_t kChunkBlocksPerSm = 3;
 constexpr uint32_t kSumChunks = 16;
-constexpr uint32_t sum_rows(uint32_t chunks) { return (chunks + kSumChunks - 1u) / kSumChunks; }
+constexpr uint32_t kSumWords = 512;
+__host__ __device__ constexpr uint32_t sum_rows(uint32_t chunks) { return (chunks + kSumChunks - 1u) / kSumChunks; }
 uint32_t chunk_pass_chunks(uint32_t n_max, int sms);
 // err: the control block's error word (bit 2: a tile copy of the scatter
 // never landed).
 void launch_chunk_pass(int bits, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
-                       uint32_t* vals_out, const uint32_t* n_ptr, int shift, uint32_t chunks, uint32_t* counts,
-                       uint32_t* sums, uint32_t* spare, uint32_t* err, cudaStream_t st);
+                       uint32_t* vals_out, const uint32_t* n_ptr, uint32_t low, int shift, uint32_t chunks,
+                       uint32_t* counts, uint32_t* sums, uint32_t* spare, uint32_t* err, cudaStream_t st);
 // Opt every sort-scatter instantiation into its shared-memory size (once per
 // device; call before any stream capture).
 void prepare_sort_kernels();

@@ -78,13 +78,19 @@ __device__ __forceinline__ void chunk_tiles(uint32_t n, uint32_t chunks, uint32_
   *t1 = (uint32_t)((uint64_t)(c + 1u) * tiles / chunks);
 }
 
+// A pass's digit of a key: BITS bits from `shift` on, of key - low for 9-bit
+// digits.
+template <int BITS>
+__device__ __forceinline__ uint32_t digit_of(uint32_t key, uint32_t low, uint32_t shift) {
+  return ((BITS > 8 ? key - low : key) >> shift) & ((1u << BITS) - 1u);
+}
+
 template <int BITS>
 __global__ void __launch_bounds__(kBlock) k_chunk_count(const uint32_t* __restrict__ keys,
-                                                        const uint32_t* __restrict__ n_ptr, int shift,
-                                                        uint32_t chunks, uint32_t* __restrict__ counts,
-                                                        uint32_t* __restrict__ sums) {
+                                                        const uint32_t* __restrict__ n_ptr, uint32_t low,
+                                                        uint32_t shift, uint32_t chunks,
+                                                        uint32_t* __restrict__ counts, uint32_t* __restrict__ sums) {
   constexpr uint32_t RADIX = 1u << BITS;
-  constexpr uint32_t MASK = RADIX - 1u;
   __shared__ uint32_t s_hist[kCountWarps][RADIX];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   for (uint32_t i = tid; i < kCountWarps * RADIX; i += kBlock) (&s_hist[0][0])[i] = 0u;
@@ -113,7 +119,7 @@ __global__ void __launch_bounds__(kBlock) k_chunk_count(const uint32_t* __restri
 #pragma unroll
     for (uint32_t q = 0; q < 16u; ++q) {
       const bool ok = s + (q >> 2) * 128u + 4u * lane + (q & 3u) < end;
-      const uint32_t d = (kk[q] >> shift) & MASK;
+      const uint32_t d = digit_of<BITS>(kk[q], low, shift);
       const uint32_t d0 = __shfl_sync(0xffffffffu, d, 0);
       if (__all_sync(0xffffffffu, ok && d == d0)) {
         if (lane == 0u) atomicAdd(&s_hist[warp][d0], 32u);
@@ -128,13 +134,16 @@ __global__ void __launch_bounds__(kBlock) k_chunk_count(const uint32_t* __restri
 #pragma unroll
     for (int w = 0; w < kCountWarps; ++w) sum += s_hist[w][d];
     counts[(size_t)blockIdx.x * RADIX + d] = sum;
-    if (sum) atomicAdd(sums + blockIdx.x / kSumChunks * RADIX + d, sum);
+    if (sum) atomicAdd(sums + blockIdx.x / kSumChunks * kSumWords + d, sum);
   }
 }
 
 // Two buffers of keys, one of values: the keys of tile t+1 stream in while
 // tile t is ranked and scattered, its values while it is ranked.
 constexpr size_t kChunkDynSmem = 3 * kSortTile * sizeof(uint32_t);
+
+// Digits owned by a thread of the scatter.
+__host__ __device__ constexpr int digits_per_thread(int bits) { return bits > 8 ? 2 : 1; }
 
 template <int BITS>
 struct ScatterShared {
@@ -212,10 +221,11 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
 // the value buffer's barrier; false if the values never landed.
 template <int BITS, bool FULL>
 __device__ __forceinline__ bool scatter_tile(ScatterShared<BITS>& sm, uint32_t* kb, uint32_t* vb, uint32_t base,
-                                             uint32_t n, int shift, uint32_t* __restrict__ keys_out,
-                                             uint32_t* __restrict__ vals_out, uint32_t& run, uint32_t parity) {
+                                             uint32_t n, uint32_t low, uint32_t shift,
+                                             uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
+                                             uint32_t (&run)[digits_per_thread(BITS)], uint32_t parity) {
   constexpr uint32_t RADIX = 1u << BITS;
-  constexpr uint32_t MASK = RADIX - 1u;
+  constexpr int D = digits_per_thread(BITS);
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t lt = (1u << lane) - 1u;
   const uint32_t wofs = warp * 32u * kSortItems;  // warp-striped: item j*32+lane of the warp's segment
@@ -226,7 +236,7 @@ __device__ __forceinline__ bool scatter_tile(ScatterShared<BITS>& sm, uint32_t* 
   for (int j = 0; j < kSortItems; ++j) {
     const bool ok = FULL || base + wofs + (uint32_t)j * 32u + lane < n;
     const uint32_t valid = FULL ? 0xffffffffu : __ballot_sync(0xffffffffu, ok);
-    const uint32_t d = (k[j] >> shift) & MASK;
+    const uint32_t d = digit_of<BITS>(k[j], low, shift);
     uint32_t peers = valid;
     if (!FULL || (j & 1)) {
       peers = match_digit<BITS>(d, valid);
@@ -250,25 +260,35 @@ __device__ __forceinline__ bool scatter_tile(ScatterShared<BITS>& sm, uint32_t* 
   }
   __syncthreads();
 
-  // Thread d: the tile's items of digit d, and with the digits below it the
-  // tile position of each warp's first item of digit d (one look-up per item
+  // Thread d: the tile's items of digit d (of digits 2d and 2d + 1 where there
+  // are more digits than threads), and with the digits below it the tile
+  // position of each warp's first item of the digit (one look-up per item
   // below).
-  uint32_t count = 0;
-  if (tid < RADIX) {
+  const bool owns = tid * D < RADIX;
+  uint32_t count[D] = {}, sum = 0;
+  if (owns) {
 #pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) count += sm.warp_hist[w][tid];
+    for (int w = 0; w < kSortWarps; ++w)
+#pragma unroll
+      for (int i = 0; i < D; ++i) count[i] += sm.warp_hist[w][tid * D + i];
   }
-  const uint32_t excl = digit_scan(count, sm.scan);
-  if (tid < RADIX) {
-    uint32_t first = excl;
 #pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) {
-      const uint32_t c = sm.warp_hist[w][tid];
-      sm.warp_hist[w][tid] = (uint16_t)first;
-      first += c;
+  for (int i = 0; i < D; ++i) sum += count[i];
+  uint32_t first = digit_scan(sum, sm.scan);
+  if (owns) {
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      sm.delta[tid * D + i] = run[i] - first;
+      run[i] += count[i];
+      uint32_t at = first;
+#pragma unroll
+      for (int w = 0; w < kSortWarps; ++w) {
+        const uint32_t c = sm.warp_hist[w][tid * D + i];
+        sm.warp_hist[w][tid * D + i] = (uint16_t)at;
+        at += c;
+      }
+      first = at;
     }
-    sm.delta[tid] = run - excl;
-    run += count;
   }
   __syncthreads();
 
@@ -277,7 +297,7 @@ __device__ __forceinline__ bool scatter_tile(ScatterShared<BITS>& sm, uint32_t* 
 #pragma unroll
   for (int j = 0; j < kSortItems; ++j) {
     if (FULL || base + wofs + (uint32_t)j * 32u + lane < n) {
-      const uint32_t d = (k[j] >> shift) & MASK;
+      const uint32_t d = digit_of<BITS>(k[j], low, shift);
       rank[j] += sm.warp_hist[warp][d];
       kb[rank[j]] = k[j];
     }
@@ -295,7 +315,7 @@ __device__ __forceinline__ bool scatter_tile(ScatterShared<BITS>& sm, uint32_t* 
 #pragma unroll 4
   for (uint32_t i = tid; i < items; i += kScatterThreads) {
     const uint32_t key = kb[i];
-    const uint32_t dst = sm.delta[(key >> shift) & MASK] + i;
+    const uint32_t dst = sm.delta[digit_of<BITS>(key, low, shift)] + i;
     keys_out[dst] = key;
     vals_out[dst] = vb[i];
   }
@@ -309,17 +329,19 @@ template <int BITS>
 __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
     k_chunk_scatter(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                     uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
-                    const uint32_t* __restrict__ n_ptr, int shift, uint32_t chunks,
+                    const uint32_t* __restrict__ n_ptr, uint32_t low, uint32_t shift, uint32_t chunks,
                     const uint32_t* __restrict__ counts, const uint32_t* __restrict__ sums,
                     uint32_t* __restrict__ spare, uint32_t* __restrict__ err) {
   constexpr uint32_t RADIX = 1u << BITS;
+  constexpr int D = digits_per_thread(BITS);
   __shared__ __align__(16) ScatterShared<BITS> sm;
   extern __shared__ uint4 s_dyn[];
   uint32_t* s_buf = reinterpret_cast<uint32_t*>(s_dyn);
 
   const uint32_t tid = threadIdx.x, c = blockIdx.x;
   // The other sums, used by the pass before this one, start the next at zero.
-  if (c < (chunks + kSumChunks - 1u) / kSumChunks && tid < 256u) spare[c * 256u + tid] = 0u;
+  if (c < sum_rows(chunks))
+    for (uint32_t i = tid; i < kSumWords; i += kScatterThreads) spare[c * kSumWords + i] = 0u;
   const uint32_t n = *n_ptr;
   uint32_t t0, t1;
   chunk_tiles(n, chunks, c, &t0, &t1);
@@ -333,24 +355,34 @@ __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
   for (uint32_t i = tid; i < kSortWarps * RADIX; i += kScatterThreads) (&sm.match[0][0])[i] = 0u;
   for (uint32_t i = tid; i < kSortWarps * RADIX * sizeof(uint16_t) / 4u; i += kScatterThreads)
     reinterpret_cast<uint32_t*>(&sm.warp_hist[0][0])[i] = 0u;
-  // Thread d: the chunk's first position of digit d: keys of the digits below
-  // it, and of its own digit in the chunks before.
-  const uint32_t group = c / kSumChunks, groups = (chunks + kSumChunks - 1u) / kSumChunks;
-  uint32_t all = 0, before = 0;
-  if (tid < RADIX) {
+  // Thread d: the chunk's first position of its digits: keys of the digits
+  // below, and of the digit itself in the chunks before.
+  const uint32_t group = c / kSumChunks, groups = sum_rows(chunks);
+  uint32_t all[D] = {}, run[D] = {}, sum = 0;
+  if (tid * D < RADIX) {
 #pragma unroll 8
-    for (uint32_t g = 0; g < groups; ++g) {
-      const uint32_t x = sums[g * RADIX + tid];
-      all += x;
-      before += g < group ? x : 0u;
-    }
+    for (uint32_t g = 0; g < groups; ++g)
+#pragma unroll
+      for (int i = 0; i < D; ++i) {
+        const uint32_t x = sums[g * kSumWords + tid * D + i];
+        all[i] += x;
+        run[i] += g < group ? x : 0u;
+      }
 #pragma unroll
     for (uint32_t r = 0; r < kSumChunks - 1u; ++r) {
       const uint32_t row = group * kSumChunks + r;
-      before += row < c ? counts[(size_t)row * RADIX + tid] : 0u;
+#pragma unroll
+      for (int i = 0; i < D; ++i) run[i] += row < c ? counts[(size_t)row * RADIX + tid * D + i] : 0u;
     }
   }
-  uint32_t run = digit_scan(all, sm.scan) + before;
+#pragma unroll
+  for (int i = 0; i < D; ++i) sum += all[i];
+  uint32_t below = digit_scan(sum, sm.scan);
+#pragma unroll
+  for (int i = 0; i < D; ++i) {
+    run[i] += below;
+    below += all[i];
+  }
 
   for (uint32_t t = t0; t < t1; ++t) {
     const uint32_t k = (t - t0) & 1u, base = t * kSortTile;
@@ -362,9 +394,9 @@ __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
     const uint32_t parity = (t - t0) & 1u;
     if (ok) {
       if ((uint64_t)base + kSortTile <= n)
-        ok = scatter_tile<BITS, true>(sm, kb, vb, base, n, shift, keys_out, vals_out, run, parity);
+        ok = scatter_tile<BITS, true>(sm, kb, vb, base, n, low, shift, keys_out, vals_out, run, parity);
       else
-        ok = scatter_tile<BITS, false>(sm, kb, vb, base, n, shift, keys_out, vals_out, run, parity);
+        ok = scatter_tile<BITS, false>(sm, kb, vb, base, n, low, shift, keys_out, vals_out, run, parity);
     } else {
       bar_wait(smem_addr(&sm.bar[2]), parity);
     }
@@ -381,10 +413,10 @@ __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
 
 template <int B>
 void launch_chunk_bits(uint32_t chunks, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
-                       uint32_t* vals_out, const uint32_t* n_ptr, int shift, uint32_t* counts, uint32_t* sums,
-                       uint32_t* spare, uint32_t* err, cudaStream_t st) {
-  k_chunk_count<B><<<chunks, kBlock, 0, st>>>(keys_in, n_ptr, shift, chunks, counts, sums);
-  k_chunk_scatter<B><<<chunks, kScatterThreads, kChunkDynSmem, st>>>(keys_in, vals_in, keys_out, vals_out, n_ptr,
+                       uint32_t* vals_out, const uint32_t* n_ptr, uint32_t low, uint32_t shift, uint32_t* counts,
+                       uint32_t* sums, uint32_t* spare, uint32_t* err, cudaStream_t st) {
+  k_chunk_count<B><<<chunks, kBlock, 0, st>>>(keys_in, n_ptr, low, shift, chunks, counts, sums);
+  k_chunk_scatter<B><<<chunks, kScatterThreads, kChunkDynSmem, st>>>(keys_in, vals_in, keys_out, vals_out, n_ptr, low,
                                                                     shift, chunks, counts, sums, spare, err);
 }
 
@@ -396,6 +428,7 @@ void configure_bits() {
 void prepare_sort_kernels() {
   configure_bits<1>(); configure_bits<2>(); configure_bits<3>(); configure_bits<4>();
   configure_bits<5>(); configure_bits<6>(); configure_bits<7>(); configure_bits<8>();
+  configure_bits<9>();
 }
 
 uint32_t chunk_pass_chunks(uint32_t n_max, int sms) {
@@ -404,11 +437,12 @@ uint32_t chunk_pass_chunks(uint32_t n_max, int sms) {
 }
 
 void launch_chunk_pass(int bits, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
-                       uint32_t* vals_out, const uint32_t* n_ptr, int shift, uint32_t chunks, uint32_t* counts,
-                       uint32_t* sums, uint32_t* spare, uint32_t* err, cudaStream_t st) {
+                       uint32_t* vals_out, const uint32_t* n_ptr, uint32_t low, int shift, uint32_t chunks,
+                       uint32_t* counts, uint32_t* sums, uint32_t* spare, uint32_t* err, cudaStream_t st) {
 #define GS_CHUNK(B)                                                                                               \
   case B:                                                                                                         \
-    launch_chunk_bits<B>(chunks, keys_in, vals_in, keys_out, vals_out, n_ptr, shift, counts, sums, spare, err, st); \
+    launch_chunk_bits<B>(chunks, keys_in, vals_in, keys_out, vals_out, n_ptr, low, (uint32_t)shift, counts, sums, \
+                         spare, err, st);                                                                         \
     break;
   switch (bits) {
     GS_CHUNK(1)
@@ -418,6 +452,7 @@ void launch_chunk_pass(int bits, const uint32_t* keys_in, const uint32_t* vals_i
     GS_CHUNK(5)
     GS_CHUNK(6)
     GS_CHUNK(7)
+    GS_CHUNK(9)
     default:
       GS_CHUNK(8)
   }
