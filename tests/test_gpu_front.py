@@ -78,6 +78,25 @@ def test_front_equals_the_oracle_and_the_separate_kernels(name):
     assert front["stats"] == again["stats"]
 
 
+@pytest.mark.parametrize("packed", [0, 1])
+@pytest.mark.parametrize("n,size,log_scale", [(2047, 16, 0.0), (2048, 16, 0.0), (2049, 16, 0.0), (1000, 1024, -4.0),
+                                              (2048, 1024, -4.0)])
+def test_both_sides_of_the_one_block_sort(n, size, log_scale, packed):
+    # All splats visible; of one tile (as many records as splats), or of 4096
+    # (two passes of the tile sort, over less and more than 2048 records).
+    scene = sc.uniform_cloud(n, seed=17, degree=0, log_scale=(log_scale, 0.1))
+    scene["means"][:, :2] = scene["means"][:, :2] % 1.0 * 0.6 + 0.05
+    frame = cam(w=size, h=size, eye=(0, 0, 20.0), depth_sort_mode=packed)
+    o = oracle.render(scene, frame, 0)
+    assert o["visible_state"][0] == n
+    assert o["state"][0] == n if size == 16 else (o["state"][0] <= 2048) == (n == 1000)
+    run = GpuRun(scene, frame, "exact", capacity=1 << 16)
+    front = run.render(frame)
+    run.close()
+    assert front["launches"] == 2
+    assert_bit_exact(front, o)
+
+
 @pytest.mark.parametrize("n", [393216, 393217])
 def test_both_sides_of_the_size_rule(n):
     scene, frame = sc.uniform_cloud(n, seed=12, degree=0, log_scale=(-4.0, 0.5)), cam(w=320, h=200)
