@@ -13,7 +13,7 @@
 // Every buffer ends up with the same contents as after the separate kernels.
 // What differs is how the stages split the work:
 //  * Compaction: the projection leaves the number of visible items of each 32
-//    (a byte); a block sums the bytes before its units, so no look-back.
+//    (a byte); a block sums the bytes before its units.
 //  * Sorts of up to 2048 items run in one block, without barriers.
 //  * Sort passes: up to a tile per block, a block ranks its tile, publishes its
 //    256 digit counts, and after a barrier sums the rows before its own; above

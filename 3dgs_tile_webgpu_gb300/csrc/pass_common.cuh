@@ -1,6 +1,6 @@
 // Shared definitions of the CUDA pass: kernel parameter blocks, the per-frame
-// control block, and the decoupled look-back protocol used by the compaction
-// and scan kernels.
+// control block, and the status words by which the chunks of the compaction
+// and scan kernels tell each other their sums.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -99,19 +99,19 @@ __device__ __forceinline__ uint32_t find_view(const uint32_t* base, uint32_t nvi
 }
 
 constexpr uint32_t kMaxSortPasses = 4;  // digit histograms held per sort
-// Persistent blocks per SM of the chunked look-back scans (compaction and
+// Persistent blocks per SM of the chunked scans (compaction and
 // ordered-count scan); scan_chunks() = their grid for n_max items.
 constexpr uint32_t kScanBlocksPerSm = 4;
 uint32_t scan_chunks(uint32_t n_max, int sms);
 
 // Per-frame control block, zeroed before each render.
 struct Control {
-  uint32_t tickets[2];           // dynamic tile ids of the look-back kernels (Ticket)
+  uint32_t tickets[2];           // dynamic chunk ids of the chunked scans (Ticket)
   uint32_t depth_hist[kMaxSortPasses][256];  // digit histograms of the fused front's chunked passes:
   uint32_t tile_hist[kMaxSortPasses][256];   // depth sort and tile sort
   uint32_t visible_state[4];     // visible, visible, radix blocks, 0
   uint32_t state[4];             // count, total, radix blocks, overflow
-  uint32_t error;                // bit 0: look-back wait or grid barrier expired; bit 2: a sort tile copy never landed
+  uint32_t error;                // bit 0: chunk-sum wait or grid barrier expired; bit 2: a sort tile copy never landed
   uint32_t pad[3];
   unsigned long long raster_stats[4];  // checked, blended, pixels, alpha-stopped
   uint32_t order_hist[34];       // raster work-list buckets (tile load classes)
@@ -121,7 +121,7 @@ struct Control {
 enum Ticket { kTicketCompact = 0, kTicketScan = 1 };
 
 // ---------------------------------------------------------------------------
-// Decoupled look-back status words: [63:34] epoch, [33:32] flag, [31:0] value.
+// Status words of the chunked scans: [63:32] epoch, [31:0] the chunk's sum.
 // A word whose epoch differs from the launch's epoch is "not yet published",
 // so the status array never needs clearing between launches. A frame's
 // launches use epochs base + 1 .. base + kEpochsPerFrame, where base is a
@@ -131,7 +131,7 @@ constexpr uint32_t kEpochsPerFrame = 16;
 
 constexpr uint32_t kSpinLimit = 1u << 22;  // default polls before a wait is declared expired (about 1 s)
 
-// The epoch of look-back launch `add` of the current frame, and how many
+// The epoch of chunked-scan launch `add` of the current frame, and how many
 // polls a wait of that launch may spend on one status word.
 struct Epoch {
   const uint32_t* base;  // device counter
@@ -140,86 +140,35 @@ struct Epoch {
   __device__ __forceinline__ uint32_t get() const { return *base + add; }
   __device__ __forceinline__ uint32_t limit() const { return spin_limit ? spin_limit : kSpinLimit; }
 };
-constexpr unsigned long long kFlagAggregate = 1ull;
-constexpr unsigned long long kFlagInclusive = 2ull;
 
-__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
+// A status word carries its value, so no other memory hangs on its order.
+__device__ __forceinline__ unsigned long long ld_status(const unsigned long long* p) {
   unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ unsigned long long pack_status(uint32_t epoch, unsigned long long flag, uint32_t value) {
-  return ((unsigned long long)epoch << 34) | (flag << 32) | (unsigned long long)value;
+__device__ __forceinline__ void st_status(unsigned long long* p, uint32_t epoch, uint32_t value) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(((unsigned long long)epoch << 32) | value)
+               : "memory");
 }
 __device__ __forceinline__ uint32_t sat_add(uint32_t a, uint32_t b) { return a + min(b, 0xffffffffu - a); }
 
-// Wait (bounded) until *p carries this launch's epoch. On expiry the error
-// word gets bit 0 and the caller treats the word as an inclusive zero, so the
+// Wait (bounded) until *p, last read as v, carries this launch's epoch; its
+// value. On expiry the error word gets bit 0 and the value is zero, so the
 // kernel always finishes and the host sees the error.
-__device__ __forceinline__ unsigned long long wait_status(const unsigned long long* p, unsigned long long v,
-                                                          uint32_t epoch, uint32_t limit, uint32_t* err,
-                                                          bool* expired) {
+__device__ __forceinline__ uint32_t wait_status(const unsigned long long* p, unsigned long long v, uint32_t epoch,
+                                                uint32_t limit, uint32_t* err) {
   uint32_t polls = 0, backoff = 8;
-  while ((uint32_t)(v >> 34) != epoch) {
+  while ((uint32_t)(v >> 32) != epoch) {
     if (++polls >= limit) {
       atomicOr(err, 1u);
-      *expired = true;
       return 0;
     }
     __nanosleep(backoff);
     backoff = backoff < 256 ? backoff * 2 : 256;
-    v = ld_acquire(p);
+    v = ld_status(p);
   }
-  return v;
-}
-
-// Warp-wide decoupled look-back for a single value per tile: every lane
-// requests K predecessors at once (lane l reads tile end - 32 k - l), so one
-// round trip covers 32 K tiles; the sub-windows are then resolved nearest
-// first, waiting only on the ones needed before an inclusive prefix turns up.
-// Returns the exclusive prefix of `tile` in every lane. All 32 lanes of the
-// warp must call it.
-template <bool SATURATE, int K = 4>
-__device__ __forceinline__ uint32_t warp_lookback(const unsigned long long* status, uint32_t tile, uint32_t epoch,
-                                                  uint32_t limit, uint32_t* err) {
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t excl = 0;
-  int64_t end = (int64_t)tile - 1;
-  while (end >= 0) {
-    unsigned long long v[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int64_t idx = end - 32 * k - (int64_t)lane;
-      v[k] = idx >= 0 ? ld_acquire(status + idx) : 0ull;
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      if (end - 32 * k < 0) return excl;  // no predecessors left
-      const int64_t idx = end - 32 * k - (int64_t)lane;
-      bool incl = true, expired = false;
-      uint32_t val = 0;
-      if (idx >= 0) {
-        const unsigned long long w = wait_status(status + idx, v[k], epoch, limit, err, &expired);
-        incl = expired || ((w >> 32) & 3ull) == kFlagInclusive;
-        val = expired ? 0u : (uint32_t)w;
-      }
-      const uint32_t inc_mask = __ballot_sync(0xffffffffu, incl);
-      const uint32_t stop = inc_mask ? (uint32_t)(__ffs(inc_mask) - 1) : 31u;  // nearest inclusive lane
-      uint32_t x = lane <= stop ? val : 0u;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, o);
-        x = SATURATE ? sat_add(x, y) : x + y;
-      }
-      excl = SATURATE ? sat_add(excl, x) : excl + x;
-      if (inc_mask) return excl;
-    }
-    end -= 32 * K;
-  }
-  return excl;
+  return (uint32_t)v;
 }
 
 // ---------------------------------------------------------------------------
@@ -268,12 +217,12 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
 // by tile, else 0), written for visible items.
 void launch_project(const BatchView& b, const PassOptions& o, float4* mean, float4* conic, float4* color,
                     uint32_t* counts, uint32_t* keys, float4* rec, float4* erec, cudaStream_t st);
-// Starts a frame: advances the look-back epoch and clears `words` words (the
+// Starts a frame: advances the epoch of the status words and clears `words` words (the
 // sorts' sums and the control block).
 void launch_frame_begin(uint32_t* epoch_base, uint32_t* zero, uint32_t words, cudaStream_t st);
 // Advance ticket counter `ticket` of the control block by one (a test hook:
-// the chunk of ticket 0 is then never scanned, so its successor's look-back
-// wait runs out).
+// the chunk of ticket 0 is then never scanned, so the waits for its
+// sum run out).
 void launch_skip_ticket(Control* ctl, uint32_t ticket, cudaStream_t st);
 void launch_compact(const uint32_t* keys, uint32_t n, uint32_t* vis_off, uint32_t* keys_out, uint32_t* vals_out,
                     Control* ctl, unsigned long long* status, Epoch epoch, uint32_t chunks, cudaStream_t st);

@@ -103,7 +103,7 @@ struct gs3d_pipeline {
   uint32_t tile_cap = 0;
   uint32_t* tile_offsets = nullptr;
   uint32_t* tile_order = nullptr;
-  // Control, output state, look-back status.
+  // Control, output state, status words of the chunked scans.
   Control* ctl = nullptr;
   uint32_t* output_state = nullptr;
   unsigned long long* status = nullptr;
@@ -126,7 +126,7 @@ struct gs3d_pipeline {
   // Layout of the last batch.
   std::vector<uint32_t> item_bases, tile_bases;
   uint32_t total_items = 0, total_tiles = 0;
-  // Device epoch counter of the look-back protocol and frames since the last
+  // Device epoch counter of the status words and frames since the last
   // status reset.
   uint32_t* epoch_dev = nullptr;
   uint64_t frames_since_reset = 0;
@@ -172,7 +172,7 @@ struct gs3d_pipeline {
   cudaEvent_t rb_event = nullptr;
   bool rb_pending = false;
   uint32_t rb_chunks = 1;
-  // Polls a look-back wait may spend on one status word (0: the default),
+  // Polls a chunk-sum wait may spend on one status word (0: the default),
   // and the test hook that withholds the compaction's first chunk.
   uint32_t wait_limit = 0;
   bool withhold_first_chunk = false;
@@ -270,7 +270,7 @@ gs3d_status validate_data(gs3d_pipeline* p, const gs3d_gaussian_data* d) {
   return GS3D_OK;
 }
 
-// Look-back status words of the compaction and the ordered-count scan: one
+// Status words of the compaction and the ordered-count scan: one
 // per chunk, at most one chunk per 256 items.
 size_t status_words_needed(uint32_t slots, uint64_t capacity) {
   (void)capacity;
@@ -771,7 +771,7 @@ void stage_batch(gs3d_pipeline* p, const gs3d_view* views, const Plan& pl, uint3
 constexpr uint32_t kFrontMaxItems = 3u << 17;
 
 // Profiled renders (events between the stages), the FP64 projection form, a
-// set wait limit and the withheld-chunk hook (both of the look-back waits,
+// set wait limit and the withheld-chunk hook (both of the chunk-sum waits,
 // which the front has none of) keep the separate kernels.
 bool use_front(const gs3d_pipeline* p, const Plan& pl) {
   return p->front_ok && pl.items > 0 && pl.items <= kFrontMaxItems && !p->profiling &&
@@ -865,7 +865,7 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
     p->last_launches = 2;
     return;
   }
-  uint32_t ep = 0;  // look-back launch index within the frame
+  uint32_t ep = 0;  // chunked-scan launch index within the frame
   auto epoch = [&]() { return Epoch{p->epoch_dev, ++ep, p->wait_limit}; };
   launch_frame_begin(p->epoch_dev, p->zeroed, 2u * p->sum_words + (uint32_t)(sizeof(Control) / sizeof(uint32_t)), st);
   launches += 1;
@@ -874,8 +874,8 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
   uint32_t* spare = p->zeroed + p->sum_words;
   if (p->withhold_first_chunk) {
     // Test hook (gs3d_pipeline_debug_withhold_chunk): the compaction's ticket
-    // counter starts at 1, so no block scans chunk 0 and the look-back of
-    // chunk 1 waits on a status word that is never published.
+    // counter starts at 1, so no block scans chunk 0 and the others wait
+    // on a status word that is never published.
     launch_skip_ticket(ctl, kTicketCompact, st);
     p->withhold_first_chunk = false;
     ++launches;

@@ -330,14 +330,14 @@ gs3d_status gs3d_pipeline_poll_stats(gs3d_pipeline* pipeline, gs3d_stats* stats,
 
 /* Failure detection (no counterpart in the reference, whose GPU waits cannot
  * hang: WebGPU has no inter-workgroup spin). The compaction and scan kernels
- * wait on their predecessors' look-back status words; a wait that spends
+ * wait on the status words of the chunks before their own; a wait that spends
  * `polls` polls (with nanosleep back-off) on one word gives up, the frame
  * reports GS3D_ERROR_DEVICE_TIMEOUT through read_stats / poll_stats, nothing
  * is left running and the pipeline stays usable. 0 restores the default of
  * 4,194,304 polls (about one second). Releases captured graphs. */
 gs3d_status gs3d_pipeline_set_wait_limit(gs3d_pipeline* pipeline, uint32_t polls);
 /* Test hook for that path: the next render's visibility compaction never
- * scans its first chunk, so the look-back of the chunk after it waits on a
+ * scans its first chunk, so the chunks after it wait on a
  * status word that nothing publishes until the wait limit runs out. The
  * render needs at least two compaction chunks (more than 256 active splats). */
 gs3d_status gs3d_pipeline_debug_withhold_chunk(gs3d_pipeline* pipeline);
