@@ -143,6 +143,7 @@ __global__ void __launch_bounds__(kBlock) k_compact(const uint32_t* __restrict__
                                                     uint32_t* __restrict__ vals_out, Control* __restrict__ ctl,
                                                     unsigned long long* __restrict__ status, Epoch ep,
                                                     uint32_t chunks) {
+  next_may_launch();
   __shared__ ScanShared sm;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   if (tid == 0) sm.chunk = atomicAdd(&ctl->tickets[kTicketCompact], 1u);

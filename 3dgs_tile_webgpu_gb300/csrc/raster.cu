@@ -11,6 +11,8 @@ __device__ __forceinline__ uint32_t load_class(uint32_t samples) { return sample
 
 __global__ void __launch_bounds__(kBlock) k_order_count(const uint32_t* __restrict__ off, uint32_t ntile,
                                                         Control* __restrict__ ctl) {
+  after_previous();
+  next_may_launch();
   __shared__ uint32_t s_hist[34];
   if (threadIdx.x < 34) s_hist[threadIdx.x] = 0u;
   __syncthreads();
@@ -25,6 +27,8 @@ __global__ void __launch_bounds__(kBlock) k_order_count(const uint32_t* __restri
 // does not depend on it).
 __global__ void __launch_bounds__(kBlock) k_order_scatter(const uint32_t* __restrict__ off, uint32_t ntile,
                                                           Control* __restrict__ ctl, uint32_t* __restrict__ order) {
+  after_previous();
+  next_may_launch();
   __shared__ uint32_t s_start[34], s_count[34], s_base[34];
   if (threadIdx.x == 0) {
     uint32_t run = 0;
@@ -53,8 +57,8 @@ void launch_tile_order(const uint32_t* tile_offsets, uint32_t ntile, Control* ct
   (void)sms;
   if (ntile == 0) return;
   const uint32_t grid = (ntile + kBlock - 1) / kBlock;
-  k_order_count<<<grid, kBlock, 0, st>>>(tile_offsets, ntile, ctl);
-  k_order_scatter<<<grid, kBlock, 0, st>>>(tile_offsets, ntile, ctl, order);
+  launch_after(k_order_count, grid, kBlock, 0, st, tile_offsets, ntile, ctl);
+  launch_after(k_order_scatter, grid, kBlock, 0, st, tile_offsets, ntile, ctl, order);
 }
 
 void launch_raster(int precision, const uint32_t* tile_offsets, const uint32_t* order, const uint32_t* ids,

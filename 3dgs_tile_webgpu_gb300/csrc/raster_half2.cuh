@@ -627,6 +627,7 @@ __global__ void __launch_bounds__(h2_threads<TILE>(), h2_min_blocks<HALF, TILE>(
                                                            const float4* __restrict__ color,
                                                            const float4* __restrict__ rec, BatchView bv,
                                                            PassOptions o, Control* __restrict__ ctl) {
+  after_previous();
   if (ctl->state[3] != 0u) return;  // overflow: nothing is published
   constexpr uint32_t PW = TILE / 8;  // patches per tile row
   __shared__ WarpStage s_stage[PW * PW];
@@ -730,6 +731,7 @@ __global__ void __launch_bounds__(hk_threads<TILE, K>(), hk_min_blocks<HALF, TIL
     k_raster_hk(const uint32_t* __restrict__ tile_offsets, const uint32_t* __restrict__ order,
                 const uint32_t* __restrict__ ids, const float4* __restrict__ mean, const float4* __restrict__ color,
                 const float4* __restrict__ rec, BatchView bv, PassOptions o, Control* __restrict__ ctl) {
+  after_previous();
   if (ctl->state[3] != 0u) return;  // overflow: nothing is published
   constexpr uint32_t PW = TILE / 8;             // patches per tile row
   constexpr uint32_t PH = TILE / (4 * K);       // patch rows per tile
@@ -828,7 +830,7 @@ inline void launch_raster_pairs_tile(const uint32_t* tile_offsets, const uint32_
                                      const float4* mean, const float4* color, const float4* rec, const BatchView& b,
                                      const PassOptions& o, Control* ctl, bool stats, cudaStream_t st) {
 #define GS_RASTER_H2(S, D)                                                                          \
-  k_raster_h2<HALF, PERIODIC, S, D, TILE><<<b.total_tiles, h2_threads<TILE>(), 0, st>>>(            \
+  launch_after(k_raster_h2<HALF, PERIODIC, S, D, TILE>, b.total_tiles, h2_threads<TILE>(), 0, st, \
       tile_offsets, order, ids, mean, color, rec, b, o, ctl)
   const bool depth = o.any_depth != 0u;
   if (stats) {
@@ -844,7 +846,7 @@ inline void launch_raster_k_tile(const uint32_t* tile_offsets, const uint32_t* o
                                  const float4* mean, const float4* color, const float4* rec, const BatchView& b,
                                  const PassOptions& o, Control* ctl, bool stats, cudaStream_t st) {
 #define GS_RASTER_HK(S, D)                                                                          \
-  k_raster_hk<HALF, PERIODIC, S, D, TILE, K><<<b.total_tiles, hk_threads<TILE, K>(), 0, st>>>(      \
+  launch_after(k_raster_hk<HALF, PERIODIC, S, D, TILE, K>, b.total_tiles, hk_threads<TILE, K>(), 0, st, \
       tile_offsets, order, ids, mean, color, rec, b, o, ctl)
   const bool depth = o.any_depth != 0u;
   if (stats) {

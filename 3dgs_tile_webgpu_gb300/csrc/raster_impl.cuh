@@ -358,6 +358,7 @@ __global__ void __launch_bounds__(TILE * TILE, TILE == 32 ? 1 : 768 / (TILE * TI
                                                    const float4* __restrict__ conic,
                                                    const float4* __restrict__ color, BatchView bv, PassOptions o,
                                                    Control* __restrict__ ctl) {
+  after_previous();
   // Overflow: the reference zeroes the raster dispatch, so nothing is written.
   if (ctl->state[3] != 0u) return;
   constexpr int NT = TILE * TILE;
@@ -448,8 +449,8 @@ void launch_raster_tile(const uint32_t* tile_offsets, const uint32_t* order, con
                         const PassOptions& o, Control* ctl, bool stats, cudaStream_t st) {
   const bool periodic = o.axis != 0u;
 #define GS_RASTER(P, S)                                                                                          \
-  k_raster<M, P, S, TILE><<<b.total_tiles, TILE * TILE, 0, st>>>(tile_offsets, order, ids, mean, conic, color, b, \
-                                                                  o, ctl)
+  launch_after(k_raster<M, P, S, TILE>, b.total_tiles, TILE * TILE, 0, st, tile_offsets, order, ids, mean,         \
+               conic, color, b, o, ctl)
   if (periodic) {
     if (stats) GS_RASTER(true, true); else GS_RASTER(true, false);
   } else {

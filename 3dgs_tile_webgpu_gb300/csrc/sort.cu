@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(kBlock) k_chunk_count(const uint32_t* __restri
                                                         const uint32_t* __restrict__ n_ptr, uint32_t low,
                                                         uint32_t shift, uint32_t chunks,
                                                         uint32_t* __restrict__ counts, uint32_t* __restrict__ sums) {
+  next_may_launch();
   constexpr uint32_t RADIX = 1u << BITS;
   __shared__ uint32_t s_hist[kCountWarps][RADIX];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -332,6 +333,7 @@ __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
                     const uint32_t* __restrict__ n_ptr, uint32_t low, uint32_t shift, uint32_t chunks,
                     const uint32_t* __restrict__ counts, const uint32_t* __restrict__ sums,
                     uint32_t* __restrict__ spare, uint32_t* __restrict__ err) {
+  after_previous();
   constexpr uint32_t RADIX = 1u << BITS;
   constexpr int D = digits_per_thread(BITS);
   __shared__ __align__(16) ScatterShared<BITS> sm;
@@ -416,8 +418,8 @@ void launch_chunk_bits(uint32_t chunks, const uint32_t* keys_in, const uint32_t*
                        uint32_t* vals_out, const uint32_t* n_ptr, uint32_t low, uint32_t shift, uint32_t* counts,
                        uint32_t* sums, uint32_t* spare, uint32_t* err, cudaStream_t st) {
   k_chunk_count<B><<<chunks, kBlock, 0, st>>>(keys_in, n_ptr, low, shift, chunks, counts, sums);
-  k_chunk_scatter<B><<<chunks, kScatterThreads, kChunkDynSmem, st>>>(keys_in, vals_in, keys_out, vals_out, n_ptr, low,
-                                                                    shift, chunks, counts, sums, spare, err);
+  launch_after(k_chunk_scatter<B>, chunks, kScatterThreads, kChunkDynSmem, st, keys_in, vals_in, keys_out, vals_out,
+               n_ptr, low, shift, chunks, counts, sums, spare, err);
 }
 
 template <int B>

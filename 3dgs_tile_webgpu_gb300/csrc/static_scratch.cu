@@ -61,6 +61,7 @@ int g_sms[kMaxDevices] = {};
 // -> 13.0 us, 100k 32.5 -> 20.1, 5M 47.8 -> 33.4 (with the chunks' sums).
 __global__ void __launch_bounds__(256) k_static_finish(Control* ctl, unsigned long long* status, uint32_t* epoch,
                                                        unsigned char* result) {
+  after_previous();
   const uint32_t tid = threadIdx.x;
   // By bytes: the words of `result` may lie at any address.
   if (tid < 8u) {
@@ -113,7 +114,7 @@ extern "C" gs3d_status gs3d_compact_visible_static(const uint32_t* keys, uint32_
   uint32_t* epoch = reinterpret_cast<uint32_t*>(scratch + kControlWords + kStatusWords);
   const uint32_t chunks = std::min<uint32_t>(scan_chunks(n, sms), (uint32_t)kStatusWords);
   launch_compact(keys, n, visible_offsets, keys_out, ids_out, ctl, status, Epoch{epoch, 1u, 0u}, chunks, st);
-  k_static_finish<<<1, 256, 0, st>>>(ctl, status, epoch, (unsigned char*)result);
+  launch_after(k_static_finish, 1, 256, 0, st, ctl, status, epoch, (unsigned char*)result);
   if (cudaGetLastError() != cudaSuccess) return GS3D_ERROR_CUDA;
   return GS3D_OK;
 }
