@@ -299,7 +299,7 @@ gs3d_status gs3d_pipeline_render_batch(gs3d_pipeline* pipeline, const gs3d_view*
                                        uint32_t attempt, int reset_valid, void* stream);
 /* Capture the batched pass for these views (scenes, sizes, targets and object
  * counts fixed) into CUDA graphs; gs3d_pipeline_launch_graph then replays it
- * with new cameras: one graph launch per frame instead of ~28 kernel launches
+ * with new cameras: one graph launch per frame instead of ~20 kernel launches
  * per launch sequence.
  * `stream` must be a non-default stream; profiling must be off. Any
  * update_data/resize_intersections drops the graphs. Two graph instances
