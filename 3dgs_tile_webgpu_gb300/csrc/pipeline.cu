@@ -595,9 +595,8 @@ struct Plan {
   uint32_t tile = kTileSize;  // pixels per tile side
   bool any_depth = false;
   // Range of the views' depths (float bits: the keys of the float32 depth
-  // sort lie in it); all of the non-negative floats in a captured graph, whose
-  // replays bring their own cameras.
-  uint32_t key_low = 0, key_high = 0x7f800000u;
+  // sort lie in it).
+  uint32_t key_low = 0, key_high = 0;
   uint32_t items = 0, tiles = 0, blocks = 0;
   size_t objects = 0;
   size_t views_off = 0, objects_off = 0, stage_bytes = 0;
@@ -783,18 +782,20 @@ bool use_front(const gs3d_pipeline* p, const Plan& pl) {
 // and the farthest far plane (near < depth < far, neither negative), so planes
 // up to a factor of 65,536 apart (0.1 to 1000: 27 bits) take three passes of 9
 // bits instead of four of 8. Stage times with four / three passes: 2M
-// ordinals (four views) 112 / 96 us, 3M 114 / 101, 6M 191 / 177; beyond the line
-// 12M 289 / 292, 12M in eight views 376 / 387, 48M 1062 / 1143, as the scatter
-// of 512 digits writes shorter runs and keeps two digits a thread.
-constexpr uint32_t kWideDigitItems = 1u << 23;
+// ordinals (four views) 112 / 85 us, 3M 114 / 92, 6M 191 / 163, 12M 283 / 250,
+// 12M in eight views 352 / 317, 48M 1006 / 945.
 struct DepthDigits {
   uint32_t low, bits, passes;
 };
-DepthDigits depth_digits(const gs3d_pipeline* p, const Plan& pl) {
+// A captured graph keeps the four passes: its replays bring other cameras.
+DepthDigits depth_digits(const gs3d_pipeline* p, const Plan& pl, cudaStream_t st) {
   if (p->desc.depth_sort_mode != GS3D_DEPTH_FLOAT32) return {0u, 8u, 2u};
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
+  if (capture != cudaStreamCaptureStatusNone) return {0u, 8u, 4u};
   const uint32_t low = pl.key_low & 0x7fffffffu;  // a near plane of -0 is 0
   const uint32_t passes = (std::max(1u, ceil_log2((uint64_t)(pl.key_high - low) + 1u)) + 8u) / 9u;
-  if (passes >= 4u || pl.items > kWideDigitItems) return {0u, 8u, 4u};
+  if (passes >= 4u) return {0u, 8u, 4u};
   return {low, 9u, passes};
 }
 
@@ -888,7 +889,7 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
   // Visibility compaction.
   mark(p, GS3D_STAGE_COMPACT, st);
   const uint32_t scan_grid = scan_chunks(N, p->sms);
-  const DepthDigits dd = depth_digits(p, pl);
+  const DepthDigits dd = depth_digits(p, pl, st);
   int cur = (int)(dd.passes & 1u);  // the sorted records end up in buffer 0
   launch_compact(p->keys, N, p->vis_off, p->dk[cur], p->dv[cur], ctl, p->status, epoch(), scan_grid, st);
   ++launches;
@@ -1055,8 +1056,6 @@ gs3d_status gs3d_pipeline_capture_graph(gs3d_pipeline* p, const gs3d_view* views
     Plan pl;
     gs3d_status s = plan_batch(p, views + k, std::min(per, count - k), &pl, batch_tile(p));
     if (s != GS3D_OK) return s;
-    pl.key_low = 0u;  // replays may bring other depth ranges
-    pl.key_high = 0x7f800000u;
     plans.push_back(pl);
     p->graph_chunks.push_back({k, pl.n, total});
     total = align16(total + pl.stage_bytes);

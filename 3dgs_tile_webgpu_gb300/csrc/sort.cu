@@ -266,29 +266,41 @@ __device__ __forceinline__ bool scatter_tile(ScatterShared<BITS>& sm, uint32_t* 
   // position of each warp's first item of the digit (one look-up per item
   // below).
   const bool owns = tid * D < RADIX;
-  uint32_t count[D] = {}, sum = 0;
-  if (owns) {
+  if constexpr (D == 1) {
+    uint32_t count = 0;
+    if (owns) {
 #pragma unroll
-    for (int w = 0; w < kSortWarps; ++w)
-#pragma unroll
-      for (int i = 0; i < D; ++i) count[i] += sm.warp_hist[w][tid * D + i];
-  }
-#pragma unroll
-  for (int i = 0; i < D; ++i) sum += count[i];
-  uint32_t first = digit_scan(sum, sm.scan);
-  if (owns) {
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-      sm.delta[tid * D + i] = run[i] - first;
-      run[i] += count[i];
-      uint32_t at = first;
+      for (int w = 0; w < kSortWarps; ++w) count += sm.warp_hist[w][tid];
+    }
+    uint32_t at = digit_scan(count, sm.scan);
+    if (owns) {
+      sm.delta[tid] = run[0] - at;
+      run[0] += count;
 #pragma unroll
       for (int w = 0; w < kSortWarps; ++w) {
-        const uint32_t c = sm.warp_hist[w][tid * D + i];
-        sm.warp_hist[w][tid * D + i] = (uint16_t)at;
+        const uint32_t c = sm.warp_hist[w][tid];
+        sm.warp_hist[w][tid] = (uint16_t)at;
         at += c;
       }
-      first = at;
+    }
+  } else {
+    // Both digits in the halves of a word (no sum of a tile passes 16 bits):
+    // half the shared accesses and half the spills of two counters per thread
+    // (6M items, three passes: 178 -> 163 us).
+    uint32_t count = 0;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) count += reinterpret_cast<const uint32_t*>(sm.warp_hist[w])[tid];
+    const uint32_t low_count = count & 0xffffu, first = digit_scan(low_count + (count >> 16), sm.scan);
+    reinterpret_cast<uint2*>(sm.delta)[tid] = make_uint2(run[0] - first, run[1] - (first + low_count));
+    run[0] += low_count;
+    run[1] += count >> 16;
+    uint32_t at = first | (first + low_count) << 16;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) {
+      uint32_t& word = reinterpret_cast<uint32_t*>(sm.warp_hist[w])[tid];
+      const uint32_t c = word;
+      word = at;
+      at += c;
     }
   }
   __syncthreads();
@@ -362,19 +374,34 @@ __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
   const uint32_t group = c / kSumChunks, groups = sum_rows(chunks);
   uint32_t all[D] = {}, run[D] = {}, sum = 0;
   if (tid * D < RADIX) {
+    // The thread's digits of row `row` of a table of rows of `words` words.
+    auto digits = [&](const uint32_t* table, uint32_t row, uint32_t words, uint32_t (&x)[D]) {
+      const uint32_t* at = table + (size_t)row * words + tid * D;
+      if constexpr (D == 2) {
+        const uint2 q = *reinterpret_cast<const uint2*>(at);
+        x[0] = q.x;
+        x[1] = q.y;
+      } else {
+        x[0] = *at;
+      }
+    };
 #pragma unroll 8
-    for (uint32_t g = 0; g < groups; ++g)
+    for (uint32_t g = 0; g < groups; ++g) {
+      uint32_t x[D];
+      digits(sums, g, kSumWords, x);
 #pragma unroll
       for (int i = 0; i < D; ++i) {
-        const uint32_t x = sums[g * kSumWords + tid * D + i];
-        all[i] += x;
-        run[i] += g < group ? x : 0u;
+        all[i] += x[i];
+        run[i] += g < group ? x[i] : 0u;
       }
+    }
 #pragma unroll
     for (uint32_t r = 0; r < kSumChunks - 1u; ++r) {
       const uint32_t row = group * kSumChunks + r;
+      uint32_t x[D] = {};
+      if (row < c) digits(counts, row, RADIX, x);
 #pragma unroll
-      for (int i = 0; i < D; ++i) run[i] += row < c ? counts[(size_t)row * RADIX + tid * D + i] : 0u;
+      for (int i = 0; i < D; ++i) run[i] += x[i];
     }
   }
 #pragma unroll

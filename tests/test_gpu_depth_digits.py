@@ -1,8 +1,8 @@
 """The digits of the depth sort's separate kernels against the oracle.
 
-Up to 8,388,608 ordinals the float32 keys are sorted by 9-bit digits of their
-distance from the nearest near plane, in as few passes as the batch's depth
-range needs, if those are fewer than the four of 8 bits. The ranges sit on
+The separate kernels sort the float32 keys by 9-bit digits of their distance
+from the nearest near plane, in as few passes as the batch's depth range
+needs, if those are fewer than the four of 8 bits. The ranges sit on
 both sides of each number of passes (9, 18 and 27 bits); the keys and ids come
 out the same for all of them. Profiled renders keep the separate kernels at
 these sizes."""
@@ -77,3 +77,33 @@ def test_views_with_their_own_ranges():
     pipe.dispose()
     for g, frame in zip(got, frames):
         assert np.array_equal(g.view(np.uint32), oracle.render(scene, frame, 0)["rgba"].view(np.uint32))
+
+
+def test_a_captured_graph_takes_every_range():
+    # Captured with planes 10 and 12 away, replayed with planes at 0 and 1e6.
+    import torch
+    from gpu_harness import dev, pipeline_options
+    n = 400_001  # beyond the fused front
+    scene = sc.uniform_cloud(n, seed=6, degree=0, log_scale=(-4.0, 0.5))
+    view = sc.look_at((0.0, 0.0, 11.0), (0.0, 0.0, 0.0))
+    captured = sc.make_frame(view, 160, 90, 55.0, 10.0, 12.0)
+    wide = dict(captured, near=0.0, far=1.0e6)
+    data = dev.DeviceScene(scene)
+    pipe = P.TiledGaussianPipeline(data.data(), pipeline_options(captured, "exact", 1 << 21))
+    color = torch.zeros((90, 160, 4), device="cuda")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    images = []
+    for frame in (captured, wide):
+        pipe.render_batch([(data.data(), P.make_camera(frame), 160, 90, color.data_ptr(), 0, "rgba32f")])
+        torch.cuda.synchronize()
+        images.append(color.cpu().numpy().copy())
+    pipe.capture_graph([(data.data(), P.make_camera(captured), 160, 90, color.data_ptr(), 0, "rgba32f")],
+                       stream.cuda_stream)
+    for frame, image in ((wide, images[1]), (captured, images[0]), (wide, images[1])):
+        pipe.launch_graph([P.make_camera(frame)], stream=stream.cuda_stream)
+        stream.synchronize()
+        assert not pipe.read_stats()["overflow"]
+        assert np.array_equal(color.cpu().numpy().view(np.uint32), image.view(np.uint32))
+    pipe.dispose()
+    assert not np.array_equal(images[0], images[1])
