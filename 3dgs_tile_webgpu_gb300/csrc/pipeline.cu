@@ -763,10 +763,10 @@ void stage_batch(gs3d_pipeline* p, const gs3d_view* views, const Plan& pl, uint3
 // Launches of up to this many ordinals take the fused front (front.cu): its
 // three blocks per SM project and sort slower than the separate kernels, but
 // it saves their launches. Frames of n ordinals at 1280x720 / 1920x1080, us,
-// front against separate kernels: 2k 69 / 164 and 78 / 176, 60k 93 / 187 and
-// 102 / 195, 200k 164 / 230 and 173 / 240, 400k 242 / 309 and 287 / 308 (with
-// a clustered scene 313 / 372 and 279 / 322), 520k 326 / 353 and 356 / 345,
-// 1M 549 / 484 and 551 / 487.
+// front against separate kernels: 2k 62 / 120 and 72 / 127, 60k 87 / 138 and
+// 100 / 149, 200k 153 / 189 and 172 / 198, 330k 197 / 229 and 210 / 241, 400k
+// 224 / 254 and 288 / 261 (with a clustered scene 277 / 289 and 258 / 258),
+// 520k 310 / 288 and 348 / 291, 1M 533 / 394 and 554 / 401.
 constexpr uint32_t kFrontMaxItems = 3u << 17;
 
 // Profiled renders (events between the stages), the FP64 projection form, a

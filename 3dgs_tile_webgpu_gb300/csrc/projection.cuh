@@ -108,8 +108,7 @@ __device__ __forceinline__ bool tile_hit(float cx, float cy, float k0, float k1,
 // otherwise (or with a centre so far out that canon is not in the period)
 // the whole axis is kept. Walking 128 columns for the 2-3 that can hit took
 // 367 us in the projection and 391 us in the emission of 400k splats at
-// 2048x1024 (of 1384 us for the frame; 391 us with this and the rasterizers'
-// fixed image per patch).
+// 2048x1024 (of 1384 us for the frame); 45 and 23 us so.
 __device__ __forceinline__ void periodic_tiles(float cen, float r, float period, int tiles, float ts, float inv,
                                                int* start, uint32_t* count, uint32_t* wrap) {
   *start = 0; *count = (uint32_t)tiles; *wrap = 0u;

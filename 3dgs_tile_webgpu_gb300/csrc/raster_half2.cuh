@@ -110,7 +110,7 @@ __device__ __forceinline__ float2 cholesky_alpha(const uint4& h, __half2 ux, __h
 // instead of boundary_delta's two divisions. *image is its index, or NaN
 // for a record whose pixels choose their image one by one (when every record
 // did, and none was culled, the rasterizer took 465 us for 400k splats at
-// 2048x1024; the whole frame takes 391 us so).
+// 2048x1024; 133 us so).
 // r0 becomes the record at the canonical centre. (wx, wy): the patch's extent
 // between its first and last pixel centres, from (x0, y0).
 __device__ __forceinline__ bool periodic_reach(float4& r0, const float4& r1, const RasterFrame& f, float x0, float y0,
