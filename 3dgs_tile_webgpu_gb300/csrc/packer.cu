@@ -103,16 +103,21 @@ __device__ __forceinline__ uint32_t pack_sh(float r, float g, float b) {
 constexpr uint32_t kPackBlock = 256;  // splats, and threads, of a block
 
 // HBM-bound: 4 (14 + 3 (C - 1)) bytes read and 28 + 4 C written per splat. A
-// block takes 256 consecutive splats: one thread per splat for the geometry,
-// then its 256 C SH words spread over the threads, so that the coefficient
-// reads (12 consecutive bytes per thread) and the word stores of a warp are
-// consecutive; with a thread per splat they lay C words apart.
+// block takes 256 consecutive splats: one thread per splat for the geometry
+// and the colour's word, then its 256 C SH words spread over the threads, so
+// that the coefficient reads (12 consecutive bytes per thread) and the word
+// stores of a warp are consecutive; with a thread per splat they lay C words
+// apart. The colour's word comes through shared memory: computed in the loop,
+// its three divisions ran in nearly every warp for two of 32 lanes. Four words
+// of a thread are in flight (2 and 8: 56 and 70 us against 60 at degree 2, 76
+// and 81 against 76 at degree 3).
 // 1M splats at degree 3: 1810 us with a thread per splat and the double
-// log1p; 92 us (3.6 TB/s) so.
+// log1p, 95 us with the words spread, 76 us (4.3 TB/s) so; 4M 322 and 261 us.
 template <uint32_t C>
 __global__ void __launch_bounds__(kPackBlock) k_pack(gs3d_splat_source src, uint32_t first,
                                                      float4* __restrict__ means, uint2* __restrict__ shape,
                                                      uint32_t* __restrict__ rot, uint32_t* __restrict__ sh) {
+  __shared__ uint32_t s_colour[kPackBlock];  // first SH words: the colours
   const uint32_t i0 = blockIdx.x * kPackBlock;
   const uint32_t count = min(kPackBlock, src.count - i0);
   if (threadIdx.x < count) {
@@ -127,21 +132,30 @@ __global__ void __launch_bounds__(kPackBlock) k_pack(gs3d_splat_source src, uint
     const float* q = src.quaternions + 4 * (size_t)i;
     const float inv = 1.0f / sqrtf(((q[0] * q[0] + q[1] * q[1]) + q[2] * q[2]) + q[3] * q[3]);
     rot[slot] = encode_oct101012(q[0] * inv, q[1] * inv, q[2] * inv, q[3] * inv);
+    const float* rgb = src.rgb + 3 * (size_t)i;
+    s_colour[threadIdx.x] =
+        pack_sh((rgb[0] - 0.5f) / kShC0, (rgb[1] - 0.5f) / kShC0, (rgb[2] - 0.5f) / kShC0);
   }
+  __syncthreads();
   uint32_t* out = sh + ((size_t)first + i0) * C;
-  const float* rgb = src.rgb + 3 * (size_t)i0;
   const float* rest = src.sh_rest + (size_t)i0 * (C - 1u) * 3u;
-#pragma unroll 4
-  for (uint32_t w = threadIdx.x; w < count * C; w += kPackBlock) {
-    const uint32_t i = w / C, k = w - i * C;  // word k of the block's splat i
-    float r, g, b;
-    if (k == 0u) {
-      r = (rgb[3u * i] - 0.5f) / kShC0; g = (rgb[3u * i + 1u] - 0.5f) / kShC0; b = (rgb[3u * i + 2u] - 0.5f) / kShC0;
-    } else {
-      const float* c = rest + (w - i - 1u) * 3u;  // (i (C - 1) + k - 1) coefficients precede it
-      r = c[0]; g = c[1]; b = c[2];
+  constexpr uint32_t kAtOnce = C < 4u ? C : 4u;  // words of a thread in flight
+  for (uint32_t w0 = threadIdx.x; w0 < count * C; w0 += kAtOnce * kPackBlock) {
+    float c[kAtOnce][3];
+#pragma unroll
+    for (uint32_t j = 0; j < kAtOnce; ++j) {
+      const uint32_t w = w0 + j * kPackBlock, i = w / C;
+      const bool read = w < count * C && w != i * C;
+      const float* at = rest + (w - i - 1u) * 3u;  // word k of splat i: i (C - 1) + k - 1 coefficients precede it
+      c[j][0] = read ? at[0] : 0.0f;
+      c[j][1] = read ? at[1] : 0.0f;
+      c[j][2] = read ? at[2] : 0.0f;
     }
-    out[w] = pack_sh(r, g, b);
+#pragma unroll
+    for (uint32_t j = 0; j < kAtOnce; ++j) {
+      const uint32_t w = w0 + j * kPackBlock, i = w / C;
+      if (w < count * C) out[w] = w == i * C ? s_colour[i] : pack_sh(c[j][0], c[j][1], c[j][2]);
+    }
   }
 }
 
