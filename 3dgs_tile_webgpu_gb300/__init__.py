@@ -307,6 +307,11 @@ class TiledGaussianPipeline:
         chunk, so the next chunk's look-back wait runs out."""
         _raise(self._lib, self._lib.gs3d_pipeline_debug_withhold_chunk(self._p), self._p)
 
+    def debug_refuse_front(self) -> None:
+        """Test hook: the next small frame's cooperative launch is refused on
+        the host; the separate kernels render it."""
+        _raise(self._lib, self._lib.gs3d_pipeline_debug_refuse_front(self._p), self._p)
+
     def read_profile(self) -> dict:
         """GaussianPassProfileStats of the last render (types.ts:105-148):
         tileLoads, appliedTileCap (None without maxRasterizedSplatsPerTile),

@@ -632,7 +632,8 @@ bool front_fits(int device) {
   static std::atomic<int> known[64];
   const bool keep = device >= 0 && device < 64;
   if (keep && known[device].load()) return known[device].load() == 2;
-  bool ok = true;
+  int cooperative = 0;
+  bool ok = cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device) == cudaSuccess && cooperative;
   for (int i = 0; i < 8; ++i) {
     int blocks = 0;
     ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, front_kernel(i & 1, i & 2, i & 4), kBlock,
@@ -644,8 +645,8 @@ bool front_fits(int device) {
   return ok;
 }
 
-void launch_front(const BatchView& b, const PassOptions& o, const FrontBuffers& w, uint32_t* frame_params,
-                  uint32_t capacity, uint32_t tile_passes, uint32_t digit_bits, int sms, cudaStream_t st) {
+cudaError_t launch_front(const BatchView& b, const PassOptions& o, const FrontBuffers& w, uint32_t* frame_params,
+                         uint32_t capacity, uint32_t tile_passes, uint32_t digit_bits, int sms, cudaStream_t st) {
   Front f;
   f.b = b;
   f.o = o;
@@ -667,8 +668,8 @@ void launch_front(const BatchView& b, const PassOptions& o, const FrontBuffers& 
   const uint32_t grid = std::min(std::max(b.total_blocks, (uint32_t)sms), kFrontBlocksPerSm * (uint32_t)sms);
   f.small_sort = std::min(grid, (uint32_t)sms) * kBlock * 4u;
   void* args[] = {&f};
-  cudaLaunchCooperativeKernel(front_kernel(b.ngroups < b.nviews, w.rec != nullptr, o.axis != 0u), dim3(grid),
-                              dim3(kBlock), args, sizeof(FrontShared), st);
+  return cudaLaunchCooperativeKernel(front_kernel(b.ngroups < b.nviews, w.rec != nullptr, o.axis != 0u), dim3(grid),
+                                     dim3(kBlock), args, sizeof(FrontShared), st);
 }
 
 }  // namespace gs

@@ -288,9 +288,11 @@ void launch_chunk_pass(int bits, const uint32_t* keys_in, const uint32_t* vals_i
 void prepare_sort_kernels();
 // The fused front of small launches (front.cu): the stages before the
 // rasterizer in one cooperative kernel of kFrontBlocksPerSm blocks per SM at
-// most. front_fits: whether all of them are resident at once on the (current)
-// device. frame_params: the staged
+// most. front_fits: whether the (current) device takes cooperative launches
+// and holds all of these blocks at once. frame_params: the staged
 // table's FrameParam words on the device. tile_order null: no work list.
+// launch_front's status: on an error nothing was enqueued (a stream or a
+// context that may use only some of the device's SMs can refuse the launch).
 constexpr uint32_t kFrontBlocksPerSm = 3;
 size_t front_scratch_words(int sms);  // words of FrontBuffers::scratch
 struct FrontBuffers {
@@ -301,8 +303,8 @@ struct FrontBuffers {
   uint32_t* output_state;
 };
 bool front_fits(int device);
-void launch_front(const BatchView& b, const PassOptions& o, const FrontBuffers& w, uint32_t* frame_params,
-                  uint32_t capacity, uint32_t tile_passes, uint32_t digit_bits, int sms, cudaStream_t st);
+cudaError_t launch_front(const BatchView& b, const PassOptions& o, const FrontBuffers& w, uint32_t* frame_params,
+                         uint32_t capacity, uint32_t tile_passes, uint32_t digit_bits, int sms, cudaStream_t st);
 // Raster work list: every tile of the batch, heaviest load class first.
 void launch_tile_order(const uint32_t* tile_offsets, uint32_t ntile, Control* ctl, uint32_t* order, int sms,
                        cudaStream_t st);

@@ -11,6 +11,7 @@
 #include <atomic>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/gs3d.h"
@@ -176,6 +177,7 @@ struct gs3d_pipeline {
   // and the test hook that withholds the compaction's first chunk.
   uint32_t wait_limit = 0;
   bool withhold_first_chunk = false;
+  bool refuse_front = false;  // test hook: the next fused front's launch fails
   // Kernel timing: one set of GS3D_STAGE_COUNT + 1 events per profiled render.
   bool profiling = false;
   std::vector<cudaEvent_t> events;  // pool, in sets of kStageEvents
@@ -858,13 +860,20 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
                             p->vis_off, {p->dk[0], p->dk[1]}, {p->dv[0], p->dv[1]}, p->ordered, p->ioff,
                             {p->tk[0], p->tk[1]}, {p->tv[0], p->tv[1]}, p->tile_offsets,
                             ordered_tiles ? p->tile_order : nullptr, p->chunk_counts, ctl, p->output_state};
-    launch_front(bv, o, w, (uint32_t*)dev, cap32, (uint32_t)tile_passes, (uint32_t)digit_bits, p->sms, st);
-    p->depth_final = 0;
-    p->tile_final = tile_passes & 1;
-    launch_raster((int)p->desc.raster_precision, p->tile_offsets, w.tile_order, p->tv[p->tile_final], p->mean,
-                  p->conic, p->color, p->rec, bv, o, ctl, p->desc.raster_stats != 0, st);
-    p->last_launches = 2;
-    return;
+    cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
+    if (!std::exchange(p->refuse_front, false))
+      e = launch_front(bv, o, w, (uint32_t*)dev, cap32, (uint32_t)tile_passes, (uint32_t)digit_bits, p->sms, st);
+    if (e == cudaSuccess) {
+      p->depth_final = 0;
+      p->tile_final = tile_passes & 1;
+      launch_raster((int)p->desc.raster_precision, p->tile_offsets, w.tile_order, p->tv[p->tile_final], p->mean,
+                    p->conic, p->color, p->rec, bv, o, ctl, p->desc.raster_stats != 0, st);
+      p->last_launches = 2;
+      return;
+    }
+    // Refused, with nothing enqueued: the separate kernels, which need no
+    // block resident beside another, take the launch.
+    cudaGetLastError();
   }
   uint32_t ep = 0;  // chunked-scan launch index within the frame
   auto epoch = [&]() { return Epoch{p->epoch_dev, ++ep, p->wait_limit}; };
@@ -1378,6 +1387,12 @@ gs3d_status gs3d_pipeline_set_wait_limit(gs3d_pipeline* p, uint32_t polls) {
 gs3d_status gs3d_pipeline_debug_withhold_chunk(gs3d_pipeline* p) {
   if (!p) return GS3D_ERROR_INVALID_ARGUMENT;
   p->withhold_first_chunk = true;
+  return GS3D_OK;
+}
+
+gs3d_status gs3d_pipeline_debug_refuse_front(gs3d_pipeline* p) {
+  if (!p) return GS3D_ERROR_INVALID_ARGUMENT;
+  p->refuse_front = true;
   return GS3D_OK;
 }
 

@@ -341,6 +341,10 @@ gs3d_status gs3d_pipeline_set_wait_limit(gs3d_pipeline* pipeline, uint32_t polls
  * status word that nothing publishes until the wait limit runs out. The
  * render needs at least two compaction chunks (more than 256 active splats). */
 gs3d_status gs3d_pipeline_debug_withhold_chunk(gs3d_pipeline* pipeline);
+/* Test hook: the cooperative launch of the next small frame's fused front
+ * fails on the host as on a stream limited to a part of the device's SMs; the
+ * separate kernels render the frame. */
+gs3d_status gs3d_pipeline_debug_refuse_front(gs3d_pipeline* pipeline);
 /* Test hook for the "allocation-failed" status (types.ts:209-233): the nth
  * device allocation the library makes from now on (1 = the next one) fails
  * as if the device were out of memory; 0 disarms. A failed workspace growth
