@@ -225,6 +225,8 @@ struct Front {
   uint32_t capacity;
   uint32_t tile_passes, digit_bits;
   uint32_t small_sort;     // most items of a pass over tiles of 1024
+  uint32_t limit;          // polls of a barrier before it expires
+  uint32_t withhold;       // test hook: block 0 leaves before the compaction
 };
 
 // Rows summed up in one row of sums: a block adds the sums of the groups
@@ -377,12 +379,14 @@ __global__ void __launch_bounds__(kBlock, kFrontBlocksPerSm) k_front(const __gri
   __shared__ unsigned long long s_sum[kFrontWarps];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, c = blockIdx.x, grid = gridDim.x;
   const uint32_t lt = (1u << lane) - 1u;
-  constexpr uint32_t limit = kSpinLimit;
+  const uint32_t limit = f.limit;
   uint32_t* barrier = f.frame + kFrameBarrier;
   uint32_t round = 0;
   auto expired = [&]() {
-    // Nothing is published: the rasterizer sees an overflowed frame, the
-    // stats the error.
+    // The rasterizer sees an overflowed frame and writes nothing, the stats
+    // see the error. (The blocks that do meet at this barrier work on data
+    // of earlier stages, all there; this block is missing at their next one,
+    // so each of them comes here.)
     if (tid == 0) {
       atomicOr(&f.ctl->error, 1u);
       atomicExch(&f.ctl->state[0], 0u);
@@ -410,6 +414,7 @@ __global__ void __launch_bounds__(kBlock, kFrontBlocksPerSm) k_front(const __gri
     __syncthreads();
   }
   GS_MEET();
+  if (f.withhold && c == 0) return;
 
   // Compaction: units of 256 items, a contiguous run per block.
   const uint32_t units = f.b.total_items / kBlock;
@@ -646,7 +651,8 @@ bool front_fits(int device) {
 }
 
 cudaError_t launch_front(const BatchView& b, const PassOptions& o, const FrontBuffers& w, uint32_t* frame_params,
-                         uint32_t capacity, uint32_t tile_passes, uint32_t digit_bits, int sms, cudaStream_t st) {
+                         uint32_t capacity, uint32_t tile_passes, uint32_t digit_bits, int sms, uint32_t wait_limit,
+                         bool withhold, cudaStream_t st) {
   Front f;
   f.b = b;
   f.o = o;
@@ -663,6 +669,8 @@ cudaError_t launch_front(const BatchView& b, const PassOptions& o, const FrontBu
   f.capacity = capacity;
   f.tile_passes = tile_passes;
   f.digit_bits = digit_bits;
+  f.limit = wait_limit ? wait_limit : kSpinLimit;
+  f.withhold = withhold ? 1u : 0u;
   // A block per projection block, at least one and at most kFrontBlocksPerSm
   // per SM (all of them resident: the blocks wait on one another).
   const uint32_t grid = std::min(std::max(b.total_blocks, (uint32_t)sms), kFrontBlocksPerSm * (uint32_t)sms);

@@ -291,6 +291,8 @@ void prepare_sort_kernels();
 // most. front_fits: whether the (current) device takes cooperative launches
 // and holds all of these blocks at once. frame_params: the staged
 // table's FrameParam words on the device. tile_order null: no work list.
+// wait_limit: polls of a barrier (0: kSpinLimit). withhold: block 0 leaves before
+// the compaction (a test hook: the others' next barrier expires).
 // launch_front's status: on an error nothing was enqueued (a stream or a
 // context that may use only some of the device's SMs can refuse the launch).
 constexpr uint32_t kFrontBlocksPerSm = 3;
@@ -304,7 +306,8 @@ struct FrontBuffers {
 };
 bool front_fits(int device);
 cudaError_t launch_front(const BatchView& b, const PassOptions& o, const FrontBuffers& w, uint32_t* frame_params,
-                         uint32_t capacity, uint32_t tile_passes, uint32_t digit_bits, int sms, cudaStream_t st);
+                         uint32_t capacity, uint32_t tile_passes, uint32_t digit_bits, int sms, uint32_t wait_limit,
+                         bool withhold, cudaStream_t st);
 // Raster work list: every tile of the batch, heaviest load class first.
 void launch_tile_order(const uint32_t* tile_offsets, uint32_t ntile, Control* ctl, uint32_t* order, int sms,
                        cudaStream_t st);

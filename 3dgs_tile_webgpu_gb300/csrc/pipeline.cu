@@ -173,7 +173,7 @@ struct gs3d_pipeline {
   cudaEvent_t rb_event = nullptr;
   bool rb_pending = false;
   uint32_t rb_chunks = 1;
-  // Polls a chunk-sum wait may spend on one status word (0: the default),
+  // Polls a wait for other blocks may spend on one word (0: the default),
   // and the test hook that withholds the compaction's first chunk.
   uint32_t wait_limit = 0;
   bool withhold_first_chunk = false;
@@ -771,12 +771,19 @@ void stage_batch(gs3d_pipeline* p, const gs3d_view* views, const Plan& pl, uint3
 // 520k 310 / 288 and 348 / 291, 1M 533 / 394 and 554 / 401.
 constexpr uint32_t kFrontMaxItems = 3u << 17;
 
-// Profiled renders (events between the stages), the FP64 projection form, a
-// set wait limit and the withheld-chunk hook (both of the chunk-sum waits,
-// which the front has none of) keep the separate kernels.
+// A barrier of the front waits for its slowest block's whole stage, some
+// microseconds to a few milliseconds, a chunk-sum wait of the separate kernels
+// for a sum that is about to come. Set wait limits below this (about 60 ms of
+// the barriers' polls) keep the kernels whose waits they were made for; a
+// working frame could run out of them in the front.
+constexpr uint32_t kFrontMinPolls = 1u << 16;
+
+// Profiled renders (events between the stages) and the FP64 projection form
+// also keep the separate kernels.
 bool use_front(const gs3d_pipeline* p, const Plan& pl) {
   return p->front_ok && pl.items > 0 && pl.items <= kFrontMaxItems && !p->profiling &&
-         p->desc.projection_precision != GS3D_PROJECTION_FP64 && p->wait_limit == 0u && !p->withhold_first_chunk;
+         p->desc.projection_precision != GS3D_PROJECTION_FP64 &&
+         (p->wait_limit == 0u || p->wait_limit >= kFrontMinPolls);
 }
 
 // Digits of the depth sort: `passes` passes of `bits` bits, of key - low where
@@ -862,8 +869,10 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
                             ordered_tiles ? p->tile_order : nullptr, p->chunk_counts, ctl, p->output_state};
     cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
     if (!std::exchange(p->refuse_front, false))
-      e = launch_front(bv, o, w, (uint32_t*)dev, cap32, (uint32_t)tile_passes, (uint32_t)digit_bits, p->sms, st);
+      e = launch_front(bv, o, w, (uint32_t*)dev, cap32, (uint32_t)tile_passes, (uint32_t)digit_bits, p->sms,
+                       p->wait_limit, p->withhold_first_chunk, st);
     if (e == cudaSuccess) {
+      p->withhold_first_chunk = false;
       p->depth_final = 0;
       p->tile_final = tile_passes & 1;
       launch_raster((int)p->desc.raster_precision, p->tile_offsets, w.tile_order, p->tv[p->tile_final], p->mean,

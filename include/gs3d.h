@@ -330,16 +330,21 @@ gs3d_status gs3d_pipeline_poll_stats(gs3d_pipeline* pipeline, gs3d_stats* stats,
 
 /* Failure detection (no counterpart in the reference, whose GPU waits cannot
  * hang: WebGPU has no inter-workgroup spin). The compaction and scan kernels
- * wait on the status words of the chunks before their own; a wait that spends
+ * wait on the status words of the chunks before their own, the blocks of small
+ * frames' fused kernel on one another at grid barriers; a wait that spends
  * `polls` polls (with nanosleep back-off) on one word gives up, the frame
  * reports GS3D_ERROR_DEVICE_TIMEOUT through read_stats / poll_stats, nothing
  * is left running and the pipeline stays usable. 0 restores the default of
- * 4,194,304 polls (about one second). Releases captured graphs. */
+ * 4,194,304 polls (one to a few seconds). A barrier waits for whole stages of
+ * the pass: under a limit below 65,536 polls small frames are rendered by the
+ * separate kernels, which take longer for them. Releases captured graphs. */
 gs3d_status gs3d_pipeline_set_wait_limit(gs3d_pipeline* pipeline, uint32_t polls);
 /* Test hook for that path: the next render's visibility compaction never
  * scans its first chunk, so the chunks after it wait on a
- * status word that nothing publishes until the wait limit runs out. The
- * render needs at least two compaction chunks (more than 256 active splats). */
+ * status word that nothing publishes until the wait limit runs out (the
+ * separate kernels need at least two compaction chunks, more than 256 active
+ * splats, for that); in the fused kernel the block of the first chunk leaves,
+ * and the others' next barrier runs out. */
 gs3d_status gs3d_pipeline_debug_withhold_chunk(gs3d_pipeline* pipeline);
 /* Test hook: the cooperative launch of the next small frame's fused front
  * fails on the host as on a stream limited to a part of the device's SMs; the

@@ -4,6 +4,11 @@ and where its blocks wait in vain, made to happen without a GPU fault.
 * A refused launch (an error code on the host, as on a stream that may use only
   a part of the device's SMs): the separate kernels render the frame. Nothing
   else may read the workspaces, which hold no frame yet.
+* A barrier that runs out: the block that compacts the first splats leaves, the
+  others give up after the set number of polls, the frame reports
+  GS3D_ERROR_DEVICE_TIMEOUT and writes no pixel, and the same pipeline renders
+  the next frame bit-exact. A limit too short for the front's barriers keeps
+  the separate kernels, whose waits it bounds (test_gpu_failures.py).
 """
 import importlib
 
@@ -58,4 +63,50 @@ def test_refused_front_in_a_captured_graph():
         run.pipe.launch_graph([cam], stream=stream.cuda_stream)
         stream.synchronize()
         assert np.array_equal(color.cpu().numpy().view(np.uint32), ref["rgba"].view(np.uint32))
+    run.close()
+
+
+LIMIT = 1 << 16  # polls: the shortest limit that the front's barriers take, some 60 ms
+
+
+def test_front_takes_set_limits_that_its_barriers_can_keep():
+    scene, frame = case(seed=93)
+    o = oracle.render(scene, frame, 0)
+    run = GpuRun(scene, frame, "exact", capacity=int(o["state"][1]) + 256)
+    for limit, front in ((0, True), (LIMIT, True), (LIMIT - 1, False), (2000, False)):
+        run.pipe.set_wait_limit(limit)
+        g = run.render(frame)
+        assert (g["launches"] == 2) == front, limit
+        assert_bit_exact(g, o)
+    run.close()
+
+
+@pytest.mark.parametrize("n", [200, 6000, 120001])  # one 256-splat unit, several, several per block
+def test_front_barrier_expires_and_pipeline_recovers(n):
+    import time
+    import torch
+    scene, frame = case(n, seed=94)
+    o = oracle.render(scene, frame, 0)
+    run = GpuRun(scene, frame, "exact", capacity=int(o["state"][1]) + 256)
+    assert_bit_exact(run.render(frame), o)
+    H, W = int(frame["height"]), int(frame["width"])
+    color = torch.full((H, W, 4), 0.25, device="cuda")
+    depth = torch.full((H, W), 0.5, device="cuda")
+    torch.cuda.synchronize()
+    run.pipe.set_wait_limit(LIMIT)
+    run.pipe.debug_withhold_chunk()
+    t0 = time.time()
+    run.pipe.render(P.make_camera(frame), color.data_ptr(), depth.data_ptr(), 7, False, "rgba32f")
+    with pytest.raises(P.GaussianPassError) as err:
+        run.pipe.read_stats()
+    assert time.time() - t0 < 30.0  # the kernel returned on its own
+    assert err.value.status == P.abi.GS3D_ERROR_DEVICE_TIMEOUT
+    assert run.pipe.last_launch_count() == 2
+    assert (color == 0.25).all() and (depth == 0.5).all()
+    # The hook applies to one render only; the next frames are complete and exact.
+    for limit in (LIMIT, 0):
+        run.pipe.set_wait_limit(limit)
+        g = run.render(frame)
+        assert g["launches"] == 2 and g["stats"]["deviceError"] == 0
+        assert_bit_exact(g, o)
     run.close()
