@@ -124,6 +124,7 @@ SIGNATURES = {
     "gs3d_pipeline_set_wait_limit": (C.c_int, [_P, C.c_uint32]),
     "gs3d_pipeline_debug_withhold_chunk": (C.c_int, [_P]),
     "gs3d_pipeline_debug_refuse_front": (C.c_int, [_P]),
+    "gs3d_debug_refuse_compact_finish": (None, []),
     "gs3d_debug_fail_allocation": (None, [C.c_uint32]),
     "gs3d_pipeline_get_resources": (C.c_int, [_P, C.POINTER(Resources)]),
     "gs3d_pipeline_read_profile": (C.c_int, [_P, C.POINTER(ProfileStats)]),

@@ -115,7 +115,7 @@ __device__ __forceinline__ void next_may_launch() { asm volatile("griddepcontrol
 
 // Launches a kernel that begins with after_previous().
 template <typename... P, typename... A>
-void launch_after(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t dynamic, cudaStream_t st, A... args) {
+cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t dynamic, cudaStream_t st, A... args) {
   cudaLaunchAttribute overlap = {};
   overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   overlap.val.programmaticStreamSerializationAllowed = 1;
@@ -126,7 +126,7 @@ void launch_after(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t dy
   config.stream = st;
   config.attrs = &overlap;
   config.numAttrs = 1;
-  cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
+  return cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
 }
 
 constexpr uint32_t kMaxSortPasses = 4;  // digit histograms held per sort

@@ -23,13 +23,16 @@
 //    call's last kernel zeroes the control block again; the status words
 //    instead carry an epoch that the same kernel advances, so a previous
 //    call's words never count as published (when the 30-bit epoch wraps, it
-//    clears the words). Calls that overlap on the GPU (two streams, or two host threads
+//    clears the words). A call whose second kernel could not be enqueued returns
+//    GS3D_ERROR_CUDA, and the next call on the device clears the whole scratch
+//    first. Calls that overlap on the GPU (two streams, or two host threads
 //    without ordering) race on the array and give wrong results: order them
 //    on one stream.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 
 #include "../../include/gs3d.h"
@@ -52,6 +55,8 @@ constexpr int kMaxDevices = 64;
 std::mutex g_mutex;
 unsigned long long* g_scratch_ptr[kMaxDevices] = {};
 int g_sms[kMaxDevices] = {};
+bool g_unfinished[kMaxDevices] = {};  // a call's compaction went out without its last kernel
+std::atomic<bool> g_refuse_finish{false};
 
 // Hands the results out and leaves the scratch ready for the next call: the
 // control block zeroed, the epoch counter advanced by one (when the 30-bit
@@ -91,6 +96,7 @@ extern "C" gs3d_status gs3d_compact_visible_static(const uint32_t* keys, uint32_
   cudaStream_t st = (cudaStream_t)stream;
   unsigned long long* scratch = nullptr;
   int sms = 1;
+  bool clear = false;
   {
     std::lock_guard<std::mutex> lock(g_mutex);
     if (!g_scratch_ptr[device]) {
@@ -108,13 +114,37 @@ extern "C" gs3d_status gs3d_compact_visible_static(const uint32_t* keys, uint32_
     }
     scratch = g_scratch_ptr[device];
     sms = g_sms[device];
+    clear = g_unfinished[device];
   }
   Control* ctl = reinterpret_cast<Control*>(scratch);
   unsigned long long* status = scratch + kControlWords;
   uint32_t* epoch = reinterpret_cast<uint32_t*>(scratch + kControlWords + kStatusWords);
+  if (clear) {
+    // The tickets of a compaction that no last kernel followed are used up and
+    // its sums carry the epoch of this call: start again from zeros. A call
+    // that is only being captured leaves that to the next one as well.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess ||
+        cudaMemsetAsync(scratch, 0, kStaticScratchWords * sizeof(unsigned long long), st) != cudaSuccess) {
+      cudaGetLastError();
+      return GS3D_ERROR_CUDA;
+    }
+    std::lock_guard<std::mutex> lock(g_mutex);
+    if (capture == cudaStreamCaptureStatusNone) g_unfinished[device] = false;
+  }
   const uint32_t chunks = std::min<uint32_t>(scan_chunks(n, sms), (uint32_t)kStatusWords);
   launch_compact(keys, n, visible_offsets, keys_out, ids_out, ctl, status, Epoch{epoch, 1u, 0u}, chunks, st);
-  launch_after(k_static_finish, 1, 256, 0, st, ctl, status, epoch, (unsigned char*)result);
+  cudaError_t finish = cudaErrorLaunchOutOfResources;
+  if (!g_refuse_finish.exchange(false))
+    finish = launch_after(k_static_finish, 1, 256, 0, st, ctl, status, epoch, (unsigned char*)result);
+  if (finish != cudaSuccess) {
+    cudaGetLastError();
+    std::lock_guard<std::mutex> lock(g_mutex);
+    g_unfinished[device] = true;
+    return GS3D_ERROR_CUDA;
+  }
   if (cudaGetLastError() != cudaSuccess) return GS3D_ERROR_CUDA;
   return GS3D_OK;
 }
+
+extern "C" void gs3d_debug_refuse_compact_finish(void) { g_refuse_finish.store(true); }

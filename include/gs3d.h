@@ -467,12 +467,16 @@ gs3d_status gs3d_pack_splats(const gs3d_splat_source* source, uint32_t first_slo
  *                      bounded device wait expired)
  * n must not exceed GS3D_STATIC_COMPACT_MAX_ITEMS (else GS3D_ERROR_RANGE);
  * keys must be 4-byte aligned. The first call on a device looks up the static
- * array's device address and the SM count. All calls share the array, which
- * keeps the previous call's contents (each call clears what must start at
- * zero): calls that overlap on the GPU race, so order them on one stream. */
+ * array's device address and the SM count. All calls share the array, and each
+ * leaves it ready for the next: calls that overlap on the GPU race, so order
+ * them on one stream. A call that returns GS3D_ERROR_CUDA writes nothing that
+ * can be relied on; the next one starts from a cleared array. */
 #define GS3D_STATIC_COMPACT_MAX_ITEMS 16777216u
 gs3d_status gs3d_compact_visible_static(const uint32_t* keys, uint32_t n, uint32_t* visible_offsets,
                                         uint32_t* keys_out, uint32_t* ids_out, uint32_t* result, void* stream);
+/* Test hook: the second kernel of the next gs3d_compact_visible_static call is
+ * not enqueued, as if its launch had failed after the first one's. */
+void gs3d_debug_refuse_compact_finish(void);
 
 /* IntersectionCapacityPolicy.next(current, demand)
  * (src/renderer/pipeline/IntersectionCapacityPolicy.ts:90-100): the capacity
