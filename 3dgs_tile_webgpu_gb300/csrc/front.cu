@@ -16,7 +16,8 @@
 //  * Sorts of up to 2048 items run in one block, without barriers.
 //  * Sort passes: up to a tile per block, a block ranks its tile, publishes its
 //    256 digit counts, and after a barrier sums the rows before its own; above
-//    that the three steps of sort.cu with barriers in between. The depth sort
+//    that a run of tiles per block, counted, and scattered after the barrier
+//    (chunk_pass). The depth sort
 //    sorts key - (smallest visible key), and passes whose digit no key has are
 //    left out (an LSD pass over equal digits moves nothing): the start buffer
 //    is chosen so that the result lands where the host expects it.
@@ -33,6 +34,7 @@
 #include "emission.cuh"
 #include "pass_common.cuh"
 #include "projection.cuh"
+#include "radix.cuh"
 
 namespace gs {
 
@@ -57,10 +59,20 @@ struct ProjectShared {
   CountShared count;
 };
 
+// The chunked passes': two buffers of keys, one of values, and the tables of a
+// tile.
+constexpr int kChunkItems = 8;
+constexpr uint32_t kChunkTile = kScatterThreads * kChunkItems;
+struct ChunkShared {
+  uint32_t keys[2][kChunkTile], vals[kChunkTile];
+  ScatterShared<8> scatter;
+};
+
 union FrontShared {
   ProjectShared project;
   TileShared<4> tile4;
   TileShared<8> tile8;
+  ChunkShared chunk;
   EmitShared emit;
 };
 
@@ -100,18 +112,6 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long v, un
   return sum;
 }
 
-// Lanes holding the same 8-bit digit.
-__device__ __forceinline__ uint32_t match_digit8(uint32_t d, uint32_t valid) {
-  uint32_t peers = valid;
-#pragma unroll
-  for (int b = 0; b < 8; ++b) {
-    const bool bit = (d >> b) & 1u;
-    const uint32_t bal = __ballot_sync(0xffffffffu, bit);
-    peers &= bit ? bal : ~bal;
-  }
-  return peers;
-}
-
 // One sort pass's parameters: digit = ((key - low) >> shift) & mask.
 struct Pass {
   const uint32_t* keys_in;
@@ -119,7 +119,6 @@ struct Pass {
   uint32_t* keys_out;
   uint32_t* vals_out;
   uint32_t n, low, shift, mask;
-  uint32_t* hist;    // chunked passes: the pass's digit histogram, zero on entry
   uint32_t* counts;  // a row of 256 per block
   uint32_t* sums;    // sums of kSumRows rows each, zero on entry
   uint32_t* spare;   // the same of the next pass, to be zeroed
@@ -149,7 +148,7 @@ __device__ __forceinline__ uint32_t rank_tile(TileShared<IPT>& sm, uint32_t* s_s
     const bool ok = first + 32u * j < p.n;
     const uint32_t valid = __ballot_sync(0xffffffffu, ok);
     const uint32_t d = p.digit(k[j]);
-    const uint32_t peers = match_digit8(d, valid);
+    const uint32_t peers = match_digit<8>(d, valid);
     const uint32_t before = __popc(peers & lt);
     uint32_t cnt = 0;
     if (ok) cnt = sm.warp_hist[warp][d];
@@ -233,6 +232,25 @@ struct Front {
 // before its own and the rows of its group, at most grid / 16 + 15 rows in all.
 constexpr uint32_t kSumRows = 16;
 
+// The global position of row c's first item of digit tid: the items of the
+// digits below, of all rows, and of the digit in the rows before.
+__device__ __forceinline__ uint32_t first_position(const Pass& p, uint32_t* s_scan, uint32_t c, uint32_t groups) {
+  const uint32_t tid = threadIdx.x, group = c / kSumRows;
+  uint32_t all = 0, before = 0, total;
+#pragma unroll 8
+  for (uint32_t g = 0; g < groups; ++g) {
+    const uint32_t x = p.sums[g * kRadix + tid];
+    all += x;
+    before += g < group ? x : 0u;
+  }
+#pragma unroll
+  for (uint32_t r = 0; r < kSumRows - 1u; ++r) {
+    const uint32_t row = group * kSumRows + r;
+    before += row < c ? p.counts[row * kRadix + tid] : 0u;
+  }
+  return block_exclusive_scan<false>(all, s_scan, &total) + before;
+}
+
 // A pass with one tile of kBlock * IPT items for each of the first blocks:
 // ranks stay in registers over the barrier. The other blocks take no part;
 // they wait at the grid's next barrier (a barrier of 98 blocks takes 0.8 us,
@@ -249,24 +267,93 @@ __device__ __forceinline__ bool tile_pass(TileShared<IPT>& sm, uint32_t* s_scan,
   if (count) atomicAdd(p.sums + c / kSumRows * kRadix + tid, count);
   if (!grid_barrier(p.barrier, ++*round * rows, limit)) return false;
   if (c < groups) p.spare[c * kRadix + tid] = 0u;
-  // Digit tid: items of all rows, and of the rows before this one.
-  uint32_t all = 0, before = 0;
-  const uint32_t group = c / kSumRows;
-#pragma unroll 8
-  for (uint32_t g = 0; g < groups; ++g) {
-    const uint32_t x = p.sums[g * kRadix + tid];
-    all += x;
-    before += g < group ? x : 0u;
-  }
-#pragma unroll
-  for (uint32_t r = 0; r < kSumRows - 1u; ++r) {
-    const uint32_t row = group * kSumRows + r;
-    before += row < c ? p.counts[row * kRadix + tid] : 0u;
-  }
-  uint32_t total;
-  sm.run[tid] = block_exclusive_scan<false>(all, s_scan, &total) + before;
+  sm.run[tid] = first_position(p, s_scan, c, groups);
   write_tile<IPT>(sm, p, c * kBlock * IPT, k, v, rank);
   return last || grid_barrier(p.barrier, ++*round * rows, limit);
+}
+
+// Asynchronous copies of the warp's own 256 items of the tile at base (those
+// below n) into buf, 16 bytes each. They go through L2, which holds what other
+// blocks wrote before the last barrier.
+__device__ __forceinline__ void load_segment(uint32_t* buf, const uint32_t* in, uint32_t base, uint32_t n) {
+  const uint32_t lane = threadIdx.x & 31u, first = (threadIdx.x >> 5) * 32u * kChunkItems + 4u * lane;
+#pragma unroll
+  for (uint32_t q = 0; q < kChunkItems / 4u; ++q) {
+    const uint32_t i = first + q * 128u;
+    if (base + i >= n) continue;
+    const uint32_t bytes = min(n - base - i, 4u) * 4u;  // the rest of the 16 becomes zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(buf + i)),
+                 "l"(in + base + i), "r"(bytes)
+                 : "memory");
+  }
+}
+// Ends a group of copies; waits for all but the last `PENDING` groups.
+__device__ __forceinline__ void end_copies() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void wait_copies() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+  __syncwarp();  // the warp reads what its other lanes copied
+}
+
+// A pass over more items than a tile of 2048 per block: each block takes a
+// contiguous run of 2048-item tiles, counts its digits, and after a barrier
+// scatters the tiles as sort.cu's kernels do (radix.cuh: the keys of the next
+// tile and the values are on their way while a tile is ranked). Tiles of 4096
+// items take 62 KB of tables instead of 37, which the other stages miss as L1,
+// and 16 items per thread spill: 300k splats at 1001x563 269 instead of 264 us,
+// 390k at 1280x720 (1.5M records) 261 instead of 251. Frames of n splats, M
+// records, us, with tiles whose loads were waited for and positions from a third
+// barrier / so: 100k at 1280x720, 1.2M 201 / 160; 390k, 4.7M 443 / 370; 200k at
+// 1920x1080, 23M 994 / 833; 20k at 3840x2160, 20M 1452 / 1181.
+__device__ __forceinline__ bool chunk_pass(ChunkShared& sm, uint32_t* s_scan, const Pass& p, uint32_t* round, bool last,
+                                           uint32_t limit) {
+  const uint32_t tid = threadIdx.x, c = blockIdx.x, groups = front_sum_rows(gridDim.x);
+  const auto digit = [&](uint32_t key) { return p.digit(key); };
+  uint32_t t0, t1;
+  chunk_tiles(p.n, kChunkTile, gridDim.x, c, &t0, &t1);
+  uint32_t(*hist)[kRadix] = sm.scatter.match;  // the counts' histograms; zero again afterwards
+  for (uint32_t i = tid; i < kFrontWarps * kRadix; i += kBlock) (&hist[0][0])[i] = 0u;
+  for (uint32_t i = tid; i < kFrontWarps * kRadix / 2u; i += kBlock)
+    reinterpret_cast<uint32_t*>(&sm.scatter.warp_hist[0][0])[i] = 0u;
+  __syncthreads();
+  count_keys<8>(hist, p.keys_in, (uint32_t)min((uint64_t)t0 * kChunkTile, (uint64_t)p.n),
+                (uint32_t)min((uint64_t)t1 * kChunkTile, (uint64_t)p.n), digit);
+  __syncthreads();
+  uint32_t count = 0;
+#pragma unroll
+  for (int w = 0; w < kFrontWarps; ++w) {
+    count += hist[w][tid];
+    hist[w][tid] = 0u;
+  }
+  p.counts[c * kRadix + tid] = count;
+  if (count) atomicAdd(p.sums + c / kSumRows * kRadix + tid, count);
+  if (!grid_barrier(p.barrier, ++*round * gridDim.x, limit)) return false;
+  if (c < groups) p.spare[c * kRadix + tid] = 0u;
+  if (t0 < t1) {
+    load_segment(sm.keys[0], p.keys_in, t0 * kChunkTile, p.n);
+    end_copies();
+    uint32_t run[1] = {first_position(p, s_scan, c, groups)};
+    for (uint32_t t = t0; t < t1; ++t) {
+      const uint32_t k = (t - t0) & 1u, base = t * kChunkTile;
+      load_segment(sm.vals, p.vals_in, base, p.n);
+      end_copies();
+      if (t + 1u < t1) load_segment(sm.keys[k ^ 1u], p.keys_in, base + kChunkTile, p.n);
+      end_copies();
+      wait_copies<2>();  // the tile's keys
+      const auto landed = [] {
+        wait_copies<1>();  // its values
+        return true;
+      };
+      if ((uint64_t)base + kChunkTile <= p.n)
+        scatter_tile<8, kChunkItems, true>(sm.scatter, sm.keys[k], sm.vals, base, p.n, digit, p.keys_out, p.vals_out,
+                                           run, landed);
+      else
+        scatter_tile<8, kChunkItems, false>(sm.scatter, sm.keys[k], sm.vals, base, p.n, digit, p.keys_out, p.vals_out,
+                                            run, landed);
+    }
+  }
+  return last || grid_barrier(p.barrier, ++*round * gridDim.x, limit);
 }
 
 // A sort of at most one tile of 2048 items (block 0 alone): the items stay in
@@ -298,74 +385,9 @@ __device__ __forceinline__ bool is_tile_pass(uint32_t n) { return n <= gridDim.x
 // A whole pass; `round` counts the sort's barriers. False: a barrier expired.
 __device__ __forceinline__ bool sort_pass(FrontShared& sm, uint32_t* s_scan, const Pass& p, uint32_t* round, bool last,
                                           uint32_t small, uint32_t limit) {
-  const uint32_t tid = threadIdx.x;
   if (p.n <= small) return tile_pass<4>(sm.tile4, s_scan, p, round, last, limit);
   if (is_tile_pass(p.n)) return tile_pass<8>(sm.tile8, s_scan, p, round, last, limit);
-  // Chunks of whole 2048-item tiles.
-  constexpr uint32_t kTile = kBlock * 8u;
-  const uint32_t tiles = (uint32_t)(((uint64_t)p.n + kTile - 1u) / kTile), per = (tiles + gridDim.x - 1u) / gridDim.x;
-  const uint32_t chunks = (tiles + per - 1u) / per;
-  const uint32_t t0 = min(blockIdx.x * per, tiles), t1 = min(t0 + per, tiles);
-  uint32_t* hist = &sm.tile8.warp_hist[0][0];
-  if (t0 < t1) {
-    for (uint32_t i = tid; i < kFrontWarps * kRadix; i += kBlock) hist[i] = 0u;
-    __syncthreads();
-    const uint32_t end = (uint32_t)min((uint64_t)t1 * kTile, (uint64_t)p.n);
-    uint32_t* mine = hist + (tid >> 5) * kRadix;
-    for (uint32_t i = t0 * kTile + 4u * tid; i < end; i += 4u * kBlock) {
-      const bool whole = i + 4u <= end;
-      const uint4 q = whole ? *reinterpret_cast<const uint4*>(p.keys_in + i)
-                            : make_uint4(p.keys_in[i], i + 1u < end ? p.keys_in[i + 1u] : 0u,
-                                         i + 2u < end ? p.keys_in[i + 2u] : 0u, 0u);
-      const uint32_t e[4] = {q.x, q.y, q.z, q.w};
-      const uint32_t lanes = __activemask();
-#pragma unroll
-      for (uint32_t x = 0; x < 4u; ++x) {
-        // A warp whose keys share a digit (common in the high digits of tile
-        // ids) adds once instead of 32 times to one address.
-        const uint32_t d = i + x < end ? p.digit(e[x]) : kRadix;
-        int same = 0;
-        __match_all_sync(lanes, d, &same);
-        if (d == kRadix) continue;
-        if (!same) atomicAdd(mine + d, 1u);
-        else if ((tid & 31u) == (uint32_t)__ffs(lanes) - 1u) atomicAdd(mine + d, (uint32_t)__popc(lanes));
-      }
-    }
-    __syncthreads();
-    uint32_t sum = 0;
-#pragma unroll
-    for (int w = 0; w < kFrontWarps; ++w) sum += hist[w * kRadix + tid];
-    p.counts[blockIdx.x * kRadix + tid] = sum;
-    if (sum) atomicAdd(p.hist + tid, sum);
-  }
-  if (!grid_barrier(p.barrier, ++*round * gridDim.x, limit)) return false;
-  for (uint32_t d = blockIdx.x; d < kRadix; d += gridDim.x) {
-    // Column d: the rows' counts become global positions.
-    uint32_t base, total;
-    block_exclusive_scan<false>(tid < d ? __ldcg(p.hist + tid) : 0u, s_scan, &base);
-    const uint32_t each = (chunks + kBlock - 1u) / kBlock, c0 = min(tid * each, chunks), c1 = min(c0 + each, chunks);
-    uint32_t local = 0;
-    for (uint32_t c = c0; c < c1; ++c) local += p.counts[c * kRadix + d];
-    uint32_t run = base + block_exclusive_scan<false>(local, s_scan, &total);
-    for (uint32_t c = c0; c < c1; ++c) {
-      const uint32_t v = p.counts[c * kRadix + d];
-      p.counts[c * kRadix + d] = run;
-      run += v;
-    }
-  }
-  if (!grid_barrier(p.barrier, ++*round * gridDim.x, limit)) return false;
-  if (t0 < t1) {
-    uint32_t run = p.counts[blockIdx.x * kRadix + tid];
-    for (uint32_t t = t0; t < t1; ++t) {
-      uint32_t k[8], v[8], rank[8];
-      const uint32_t count = rank_tile<8>(sm.tile8, s_scan, p, t * kTile, k, v, rank);
-      sm.tile8.run[tid] = run;
-      write_tile<8>(sm.tile8, p, t * kTile, k, v, rank);
-      run += count;
-      __syncthreads();  // the tile's shared memory is free again
-    }
-  }
-  return last || grid_barrier(p.barrier, ++*round * gridDim.x, limit);
+  return chunk_pass(sm.chunk, s_scan, p, round, last, limit);
 }
 
 // Class of a tile in the raster work list, as raster.cu's.
@@ -473,12 +495,12 @@ __global__ void __launch_bounds__(kBlock, kFrontBlocksPerSm) k_front(const __gri
       if (stage < passes) {
         const bool one = odd != ((stage & 1u) != 0u);  // buffer 1 to buffer 0
         p = {one ? f.dk1 : f.dk0, one ? f.dv1 : f.dv0, one ? f.dk0 : f.dk1, one ? f.dv0 : f.dv1, visible, low,
-             8u * stage, 255u, f.ctl->depth_hist[stage], f.scratch, sums, spare, f.frame + kFrameDepthBarrier};
+             8u * stage, 255u, f.scratch, sums, spare, f.frame + kFrameDepthBarrier};
       } else {
         const uint32_t pass = stage - passes - 1u;
         const bool one = pass & 1u;
         p = {one ? f.tk1 : f.tk0, one ? f.tv1 : f.tv0, one ? f.tk0 : f.tk1, one ? f.tv0 : f.tv1, count, 0u,
-             f.digit_bits * pass, (1u << f.digit_bits) - 1u, f.ctl->tile_hist[pass], f.scratch, sums, spare,
+             f.digit_bits * pass, (1u << f.digit_bits) - 1u, f.scratch, sums, spare,
              f.frame + kFrameTileBarrier};
       }
       const bool last = stage + 1u == passes || stage == passes + f.tile_passes;
@@ -501,11 +523,9 @@ __global__ void __launch_bounds__(kBlock, kFrontBlocksPerSm) k_front(const __gri
         GS_MEET();
         sort_round = 0;
       }
-      if (is_tile_pass(p.n)) {  // its sums are used, the spare ones zeroed
-        uint32_t* used = sums;
-        sums = spare;
-        spare = used;
-      }
+      uint32_t* used = sums;  // the spare ones are zeroed
+      sums = spare;
+      spare = used;
       continue;
     }
     // Tile counts in depth order and their saturating scan: runs of whole

@@ -129,7 +129,7 @@ cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, uint32_t block, si
   return cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
 }
 
-constexpr uint32_t kMaxSortPasses = 4;  // digit histograms held per sort
+constexpr uint32_t kMaxSortPasses = 4;  // passes of a tile sort
 // Persistent blocks per SM of the chunked scans (compaction and
 // ordered-count scan); scan_chunks() = their grid for n_max items.
 constexpr uint32_t kScanBlocksPerSm = 4;
@@ -138,8 +138,6 @@ uint32_t scan_chunks(uint32_t n_max, int sms);
 // Per-frame control block, zeroed before each render.
 struct Control {
   uint32_t tickets[2];           // dynamic chunk ids of the chunked scans (Ticket)
-  uint32_t depth_hist[kMaxSortPasses][256];  // digit histograms of the fused front's chunked passes:
-  uint32_t tile_hist[kMaxSortPasses][256];   // depth sort and tile sort
   uint32_t visible_state[4];     // visible, visible, radix blocks, 0
   uint32_t state[4];             // count, total, radix blocks, overflow
   uint32_t error;                // bit 0: chunk-sum wait or grid barrier expired; bit 2: a sort tile copy never landed

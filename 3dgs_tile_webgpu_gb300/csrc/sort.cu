@@ -49,41 +49,22 @@
 #include <algorithm>
 
 #include "pass_common.cuh"
+#include "radix.cuh"
 
 namespace gs {
 
-constexpr int kCountWarps = kBlock / 32;
-constexpr int kScatterThreads = 256;
-constexpr int kSortWarps = kScatterThreads / 32;
 constexpr int kSortItems = 16;  // kSortTile = 8 warps * 32 lanes * 16 items
 static_assert(kSortTile == (uint32_t)(kScatterThreads * kSortItems), "a tile is 16 items per thread");
-
-// Lanes of the warp holding the same BITS-bit digit, by ballot bit-splitting.
-template <int BITS>
-__device__ __forceinline__ uint32_t match_digit(uint32_t d, uint32_t valid_mask) {
-  uint32_t peers = valid_mask;
-#pragma unroll
-  for (int b = 0; b < BITS; ++b) {
-    const bool bit = (d >> b) & 1u;
-    const uint32_t bal = __ballot_sync(0xffffffffu, bit);
-    peers &= bit ? bal : ~bal;
-  }
-  return peers;
-}
-
-// Tiles [t0, t1) of chunk c when n items split over `chunks` chunks.
-__device__ __forceinline__ void chunk_tiles(uint32_t n, uint32_t chunks, uint32_t c, uint32_t* t0, uint32_t* t1) {
-  const uint32_t tiles = (uint32_t)(((uint64_t)n + kSortTile - 1) / kSortTile);
-  *t0 = (uint32_t)((uint64_t)c * tiles / chunks);
-  *t1 = (uint32_t)((uint64_t)(c + 1u) * tiles / chunks);
-}
 
 // A pass's digit of a key: BITS bits from `shift` on, of key - low for 9-bit
 // digits.
 template <int BITS>
-__device__ __forceinline__ uint32_t digit_of(uint32_t key, uint32_t low, uint32_t shift) {
-  return ((BITS > 8 ? key - low : key) >> shift) & ((1u << BITS) - 1u);
-}
+struct PassDigit {
+  uint32_t low, shift;
+  __device__ __forceinline__ uint32_t operator()(uint32_t key) const {
+    return ((BITS > 8 ? key - low : key) >> shift) & ((1u << BITS) - 1u);
+  }
+};
 
 template <int BITS>
 __global__ void __launch_bounds__(kBlock) k_chunk_count(const uint32_t* __restrict__ keys,
@@ -93,42 +74,15 @@ __global__ void __launch_bounds__(kBlock) k_chunk_count(const uint32_t* __restri
   next_may_launch();
   constexpr uint32_t RADIX = 1u << BITS;
   __shared__ uint32_t s_hist[kCountWarps][RADIX];
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t tid = threadIdx.x;
   for (uint32_t i = tid; i < kCountWarps * RADIX; i += kBlock) (&s_hist[0][0])[i] = 0u;
   __syncthreads();
   const uint32_t n = *n_ptr;
   uint32_t t0, t1;
-  chunk_tiles(n, chunks, blockIdx.x, &t0, &t1);
+  chunk_tiles(n, kSortTile, chunks, blockIdx.x, &t0, &t1);
   const uint32_t begin = (uint32_t)min((uint64_t)t0 * kSortTile, (uint64_t)n);
   const uint32_t end = (uint32_t)min((uint64_t)t1 * kSortTile, (uint64_t)n);
-  // Each warp takes 512-key runs: four 16-byte loads per lane in flight
-  // before any counting (begin is a multiple of 4096, so they are aligned).
-  constexpr uint32_t kRun = 512u;
-  for (uint32_t s = begin + warp * kRun; s < end; s += kCountWarps * kRun) {
-    uint32_t kk[16];
-#pragma unroll
-    for (uint32_t q = 0; q < 4u; ++q) {
-      const uint32_t i0 = s + q * 128u + 4u * lane;
-      if (i0 + 4u <= end) {
-        const uint4 v = *reinterpret_cast<const uint4*>(keys + i0);
-        kk[4 * q] = v.x; kk[4 * q + 1] = v.y; kk[4 * q + 2] = v.z; kk[4 * q + 3] = v.w;
-      } else {
-#pragma unroll
-        for (uint32_t e = 0; e < 4u; ++e) kk[4 * q + e] = i0 + e < end ? keys[i0 + e] : 0u;
-      }
-    }
-#pragma unroll
-    for (uint32_t q = 0; q < 16u; ++q) {
-      const bool ok = s + (q >> 2) * 128u + 4u * lane + (q & 3u) < end;
-      const uint32_t d = digit_of<BITS>(kk[q], low, shift);
-      const uint32_t d0 = __shfl_sync(0xffffffffu, d, 0);
-      if (__all_sync(0xffffffffu, ok && d == d0)) {
-        if (lane == 0u) atomicAdd(&s_hist[warp][d0], 32u);
-      } else if (ok) {
-        atomicAdd(&s_hist[warp][d], 1u);
-      }
-    }
-  }
+  count_keys<BITS>(s_hist, keys, begin, end, PassDigit<BITS>{low, shift});
   __syncthreads();
   for (uint32_t d = tid; d < RADIX; d += kBlock) {
     uint32_t sum = 0;
@@ -142,36 +96,6 @@ __global__ void __launch_bounds__(kBlock) k_chunk_count(const uint32_t* __restri
 // Two buffers of keys, one of values: the keys of tile t+1 stream in while
 // tile t is ranked and scattered, its values while it is ranked.
 constexpr size_t kChunkDynSmem = 3 * kSortTile * sizeof(uint32_t);
-
-// Digits owned by a thread of the scatter.
-__host__ __device__ constexpr int digits_per_thread(int bits) { return bits > 8 ? 2 : 1; }
-
-template <int BITS>
-struct ScatterShared {
-  uint16_t warp_hist[kSortWarps][1u << BITS];  // a warp's items per digit, then its first tile position
-  uint32_t match[kSortWarps][1u << BITS];  // lanes of the warp's current row holding each digit; zero in between
-  uint32_t delta[1u << BITS];  // global position of the tile's item i of a digit, minus i
-  uint32_t scan[8];
-  unsigned long long bar[3];  // bulk-copy completion of the two key buffers and the value buffer
-};
-
-// Exclusive scan of one value per digit over the threads below 256, in two
-// block barriers; every thread of the block calls it.
-__device__ __forceinline__ uint32_t digit_scan(uint32_t v, uint32_t* s_scan) {
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  uint32_t x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= (uint32_t)o) x += y;
-  }
-  if (lane == 31u && warp < 8u) s_scan[warp] = x;
-  __syncthreads();
-  uint32_t before = 0;
-#pragma unroll
-  for (uint32_t w = 0; w < 7u; ++w) before += w < warp ? s_scan[w] : 0u;
-  return before + x - v;
-}
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -214,130 +138,6 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
   return false;
 }
 
-// Ranks the tile held in kb/vb (items base .. base + 4096, those below n),
-// stages it in place in block-sorted order and writes each digit's run to its
-// global position. FULL: every item of the tile is below n. `run`: the global
-// position of the next item of digit threadIdx.x (threads below 2^BITS).
-// Leaves warp_hist zeroed and run advanced past the tile. parity: the phase of
-// the value buffer's barrier; false if the values never landed.
-template <int BITS, bool FULL>
-__device__ __forceinline__ bool scatter_tile(ScatterShared<BITS>& sm, uint32_t* kb, uint32_t* vb, uint32_t base,
-                                             uint32_t n, uint32_t low, uint32_t shift,
-                                             uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
-                                             uint32_t (&run)[digits_per_thread(BITS)], uint32_t parity) {
-  constexpr uint32_t RADIX = 1u << BITS;
-  constexpr int D = digits_per_thread(BITS);
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  const uint32_t lt = (1u << lane) - 1u;
-  const uint32_t wofs = warp * 32u * kSortItems;  // warp-striped: item j*32+lane of the warp's segment
-  uint32_t k[kSortItems], rank[kSortItems];
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) k[j] = kb[wofs + (uint32_t)j * 32u + lane];
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    const bool ok = FULL || base + wofs + (uint32_t)j * 32u + lane < n;
-    const uint32_t valid = FULL ? 0xffffffffu : __ballot_sync(0xffffffffu, ok);
-    const uint32_t d = digit_of<BITS>(k[j], low, shift);
-    uint32_t peers = valid;
-    if (!FULL || (j & 1)) {
-      peers = match_digit<BITS>(d, valid);
-    } else if (!__all_sync(0xffffffffu, d == __shfl_sync(0xffffffffu, d, 0))) {
-      // Each lane sets its bit in its digit's word; one digit for the whole
-      // row would serialise the 32 atomics and needs none.
-      atomicOr(&sm.match[warp][d], 1u << lane);
-      __syncwarp();
-      peers = sm.match[warp][d];
-    }
-    const uint32_t before = __popc(peers & lt);
-    uint32_t cnt = 0;
-    if (ok) cnt = sm.warp_hist[warp][d];
-    rank[j] = cnt + before;
-    __syncwarp();
-    if (ok && before == 0) {
-      sm.warp_hist[warp][d] = (uint16_t)(cnt + __popc(peers));
-      if (FULL && !(j & 1)) sm.match[warp][d] = 0u;
-    }
-    __syncwarp();
-  }
-  __syncthreads();
-
-  // Thread d: the tile's items of digit d (of digits 2d and 2d + 1 where there
-  // are more digits than threads), and with the digits below it the tile
-  // position of each warp's first item of the digit (one look-up per item
-  // below).
-  const bool owns = tid * D < RADIX;
-  if constexpr (D == 1) {
-    uint32_t count = 0;
-    if (owns) {
-#pragma unroll
-      for (int w = 0; w < kSortWarps; ++w) count += sm.warp_hist[w][tid];
-    }
-    uint32_t at = digit_scan(count, sm.scan);
-    if (owns) {
-      sm.delta[tid] = run[0] - at;
-      run[0] += count;
-#pragma unroll
-      for (int w = 0; w < kSortWarps; ++w) {
-        const uint32_t c = sm.warp_hist[w][tid];
-        sm.warp_hist[w][tid] = (uint16_t)at;
-        at += c;
-      }
-    }
-  } else {
-    // Both digits in the halves of a word (no sum of a tile passes 16 bits):
-    // half the shared accesses and half the spills of two counters per thread
-    // (6M items, three passes: 178 -> 163 us).
-    uint32_t count = 0;
-#pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) count += reinterpret_cast<const uint32_t*>(sm.warp_hist[w])[tid];
-    const uint32_t low_count = count & 0xffffu, first = digit_scan(low_count + (count >> 16), sm.scan);
-    reinterpret_cast<uint2*>(sm.delta)[tid] = make_uint2(run[0] - first, run[1] - (first + low_count));
-    run[0] += low_count;
-    run[1] += count >> 16;
-    uint32_t at = first | (first + low_count) << 16;
-#pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) {
-      uint32_t& word = reinterpret_cast<uint32_t*>(sm.warp_hist[w])[tid];
-      const uint32_t c = word;
-      word = at;
-      at += c;
-    }
-  }
-  __syncthreads();
-
-  // Keys first (every raw key is in registers), then the values (read raw
-  // into the keys' registers, then written once every thread has read).
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) {
-    if (FULL || base + wofs + (uint32_t)j * 32u + lane < n) {
-      const uint32_t d = digit_of<BITS>(k[j], low, shift);
-      rank[j] += sm.warp_hist[warp][d];
-      kb[rank[j]] = k[j];
-    }
-  }
-  const bool landed = bar_wait(smem_addr(&sm.bar[2]), parity);
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j) k[j] = vb[wofs + (uint32_t)j * 32u + lane];
-  if (!__syncthreads_and(landed)) return false;
-#pragma unroll
-  for (int j = 0; j < kSortItems; ++j)
-    if (FULL || base + wofs + (uint32_t)j * 32u + lane < n) vb[rank[j]] = k[j];
-  __syncthreads();
-
-  const uint32_t items = FULL ? kSortTile : min(kSortTile, n - base);
-#pragma unroll 4
-  for (uint32_t i = tid; i < items; i += kScatterThreads) {
-    const uint32_t key = kb[i];
-    const uint32_t dst = sm.delta[digit_of<BITS>(key, low, shift)] + i;
-    keys_out[dst] = key;
-    vals_out[dst] = vb[i];
-  }
-  for (uint32_t i = tid; i < kSortWarps * RADIX * sizeof(uint16_t) / 4u; i += kScatterThreads)
-    reinterpret_cast<uint32_t*>(&sm.warp_hist[0][0])[i] = 0u;
-  __syncthreads();
-  return true;
-}
-
 template <int BITS>
 __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
     k_chunk_scatter(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
@@ -349,6 +149,7 @@ __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
   constexpr uint32_t RADIX = 1u << BITS;
   constexpr int D = digits_per_thread(BITS);
   __shared__ __align__(16) ScatterShared<BITS> sm;
+  __shared__ unsigned long long s_bar[3];  // bulk-copy completion of the two key buffers and the value buffer
   extern __shared__ uint4 s_dyn[];
   uint32_t* s_buf = reinterpret_cast<uint32_t*>(s_dyn);
 
@@ -358,14 +159,14 @@ __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
     for (uint32_t i = tid; i < kSumWords; i += kScatterThreads) spare[c * kSumWords + i] = 0u;
   const uint32_t n = *n_ptr;
   uint32_t t0, t1;
-  chunk_tiles(n, chunks, c, &t0, &t1);
+  chunk_tiles(n, kSortTile, chunks, c, &t0, &t1);
   if (t0 >= t1) return;
-  if (tid < 3u) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sm.bar[tid])) : "memory");
+  if (tid < 3u) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s_bar[tid])) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncthreads();
   uint32_t phases = 0;  // parity of the next phase of each buffer's barrier
   uint32_t* vb = s_buf + 2u * kSortTile;
-  load_tile_bulk(keys_in, t0 * kSortTile, n, s_buf, smem_addr(&sm.bar[0]));
+  load_tile_bulk(keys_in, t0 * kSortTile, n, s_buf, smem_addr(&s_bar[0]));
   for (uint32_t i = tid; i < kSortWarps * RADIX; i += kScatterThreads) (&sm.match[0][0])[i] = 0u;
   for (uint32_t i = tid; i < kSortWarps * RADIX * sizeof(uint16_t) / 4u; i += kScatterThreads)
     reinterpret_cast<uint32_t*>(&sm.warp_hist[0][0])[i] = 0u;
@@ -416,25 +217,27 @@ __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
   for (uint32_t t = t0; t < t1; ++t) {
     const uint32_t k = (t - t0) & 1u, base = t * kSortTile;
     uint32_t* kb = s_buf + k * kSortTile;
-    load_tile_bulk(vals_in, base, n, vb, smem_addr(&sm.bar[2]));
+    load_tile_bulk(vals_in, base, n, vb, smem_addr(&s_bar[2]));
     if (t + 1u < t1)
-      load_tile_bulk(keys_in, base + kSortTile, n, s_buf + (k ^ 1u) * kSortTile, smem_addr(&sm.bar[k ^ 1u]));
-    bool ok = __syncthreads_and(bar_wait(smem_addr(&sm.bar[k]), (phases >> k) & 1u));
+      load_tile_bulk(keys_in, base + kSortTile, n, s_buf + (k ^ 1u) * kSortTile, smem_addr(&s_bar[k ^ 1u]));
+    bool ok = __syncthreads_and(bar_wait(smem_addr(&s_bar[k]), (phases >> k) & 1u));
     const uint32_t parity = (t - t0) & 1u;
     if (ok) {
+      const PassDigit<BITS> digit = {low, shift};
+      auto landed = [&] { return bar_wait(smem_addr(&s_bar[2]), parity); };
       if ((uint64_t)base + kSortTile <= n)
-        ok = scatter_tile<BITS, true>(sm, kb, vb, base, n, low, shift, keys_out, vals_out, run, parity);
+        ok = scatter_tile<BITS, kSortItems, true>(sm, kb, vb, base, n, digit, keys_out, vals_out, run, landed);
       else
-        ok = scatter_tile<BITS, false>(sm, kb, vb, base, n, low, shift, keys_out, vals_out, run, parity);
+        ok = scatter_tile<BITS, kSortItems, false>(sm, kb, vb, base, n, digit, keys_out, vals_out, run, landed);
     } else {
-      bar_wait(smem_addr(&sm.bar[2]), parity);
+      bar_wait(smem_addr(&s_bar[2]), parity);
     }
     phases ^= 1u << k;
     if (!ok) {
       // A copy never landed: flag the frame and leave, after the copy of the
       // next keys (if one was issued) had its own bounded wait.
       if (tid == 0) atomicOr(err, 4u);
-      if (t + 1u < t1) bar_wait(smem_addr(&sm.bar[k ^ 1u]), (phases >> (k ^ 1u)) & 1u);
+      if (t + 1u < t1) bar_wait(smem_addr(&s_bar[k ^ 1u]), (phases >> (k ^ 1u)) & 1u);
       return;
     }
   }

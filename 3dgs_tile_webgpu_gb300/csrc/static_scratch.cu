@@ -10,7 +10,7 @@
 // per-call control block and the epoch counter) lives in the fixed
 // device array below instead of memory allocated per pipeline.
 //
-// Cost of the array: kStaticScratchWords * 8 bytes (about 41 KB), held on
+// Cost of the array: kStaticScratchWords * 8 bytes (about 33 KB), held on
 // every GPU that loads the library until the process exits.
 //
 // Rules for callers:

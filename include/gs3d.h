@@ -459,7 +459,7 @@ gs3d_status gs3d_pack_splats(const gs3d_splat_source* source, uint32_t first_slo
  * own arena or allocator (and must not see allocations they did not make),
  * and real-time loops that must not stall on the driver's allocator. The
  * caller passes every input and output; the kernel's scratch is a static
- * device array of about 41 KB per GPU, held until the process exits.
+ * device array of about 33 KB per GPU, held until the process exits.
  *   keys[n]            per-ordinal depth key, 0xffffffff = not visible
  *   visible_offsets[n] exclusive count of visible ordinals before each one
  *   keys_out/ids_out   (key, ordinal) of the visible ordinals, in ordinal order
