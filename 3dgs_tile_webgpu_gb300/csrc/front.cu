@@ -691,9 +691,10 @@ cudaError_t launch_front(const BatchView& b, const PassOptions& o, const FrontBu
   f.digit_bits = digit_bits;
   f.limit = wait_limit ? wait_limit : kSpinLimit;
   f.withhold = withhold ? 1u : 0u;
-  // A block per projection block, at least one and at most kFrontBlocksPerSm
-  // per SM (all of them resident: the blocks wait on one another).
-  const uint32_t grid = std::min(std::max(b.total_blocks, (uint32_t)sms), kFrontBlocksPerSm * (uint32_t)sms);
+  // A block per 256 ordinals (the views of a group share projection blocks, but
+  // no later stage), at least one and at most kFrontBlocksPerSm per SM (all of
+  // them resident: the blocks wait on one another).
+  const uint32_t grid = std::min(std::max(b.total_items / kBlock, (uint32_t)sms), kFrontBlocksPerSm * (uint32_t)sms);
   f.small_sort = std::min(grid, (uint32_t)sms) * kBlock * 4u;
   void* args[] = {&f};
   return cudaLaunchCooperativeKernel(front_kernel(b.ngroups < b.nviews, w.rec != nullptr, o.axis != 0u), dim3(grid),

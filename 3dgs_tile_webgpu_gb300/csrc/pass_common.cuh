@@ -234,6 +234,8 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
   return excl;
 }
 
+constexpr uint32_t kProjectBlocksPerSm = 4;  // resident blocks of the projection kernel
+
 // Launch wrappers implemented in the .cu files.
 // Packed raster record of a visible splat, read by the fast raster forms with
 // one 32-byte gather (two float4, 32-byte aligned):

@@ -20,10 +20,10 @@ namespace gs {
 // The projection kernel: a block per 256 ordinals of a view group
 // (project_block, projection.cuh).
 template <bool FP64, bool GROUPED, bool FAST_SH, bool PERIODIC>
-__global__ void __launch_bounds__(kBlock, 4) k_project(BatchView b, PassOptions o, float4* __restrict__ mean_out,
-                                                    float4* __restrict__ conic_out, float4* __restrict__ color_out,
-                                                    uint32_t* __restrict__ count_out, uint32_t* __restrict__ key_out,
-                                                    float4* __restrict__ rec_out, float4* __restrict__ erec_out) {
+__global__ void __launch_bounds__(kBlock, kProjectBlocksPerSm)
+    k_project(BatchView b, PassOptions o, float4* __restrict__ mean_out, float4* __restrict__ conic_out,
+              float4* __restrict__ color_out, uint32_t* __restrict__ count_out, uint32_t* __restrict__ key_out,
+              float4* __restrict__ rec_out, float4* __restrict__ erec_out) {
   __shared__ float s_snorm[256];
   __shared__ uint32_t s_group;
   __shared__ CountShared s_count;

@@ -625,12 +625,19 @@ bool same_scene(const gs3d_view& a, const gs3d_view& b) {
          x.sh_degree == y.sh_degree;
 }
 
+// Most views of a group, for a scene of `blocks` projection blocks in a batch of
+// n views: a block projects the group's views one after the other, so a small
+// scene's views are spread over as many groups as fill the SMs.
+uint32_t group_views(const gs3d_pipeline* p, uint64_t blocks, uint32_t n) {
+  return (uint32_t)std::max<uint64_t>(1, blocks * n / (kProjectBlocksPerSm * (uint64_t)p->sms));
+}
+
 // Validate a batch, grow every workspace it needs and lay out its batch
 // table. Not capturable (it may allocate).
 gs3d_status plan_batch(gs3d_pipeline* p, const gs3d_view* views, uint32_t n, Plan* out, uint32_t tile) {
   if (n == 0 || n > kMaxViews) return fail(p, GS3D_ERROR_RANGE, "a batch holds 1 to 4096 views");
   uint64_t items = 0, tiles = 0, blocks = 0;
-  uint32_t ngroups = 0;
+  uint32_t ngroups = 0, in_group = 0;
   bool any_depth = false;
   size_t objects = 0;
   float near = INFINITY, far = 0.0f;
@@ -652,10 +659,12 @@ gs3d_status plan_batch(gs3d_pipeline* p, const gs3d_view* views, uint32_t n, Pla
     // TiledGaussianPipeline.ts:294-296
     if (tx > 65535u || ty > 65535u) return fail(p, GS3D_ERROR_RANGE, "Render size exceeds WebGPU's tile dispatch limit");
     const uint64_t b = ((uint64_t)v.data->active_count + kBlock - 1) / kBlock;
-    if (i == 0 || !same_scene(views[i - 1], v)) {
+    if (i == 0 || !same_scene(views[i - 1], v) || in_group == group_views(p, b, n)) {
       blocks += b;
       ++ngroups;
+      in_group = 0;
     }
+    ++in_group;
     items += b * kBlock;
     tiles += (uint64_t)tx * ty;
     objects += v.camera->object_count;
@@ -699,7 +708,7 @@ void stage_batch(gs3d_pipeline* p, const gs3d_view* views, const Plan& pl, uint3
   uint32_t* h_tile = h_item + (n + 1);
   uint32_t* h_gblock = h_tile + (n + 1);
   uint32_t* h_gview = h_gblock + (n + 1);
-  uint32_t ngroups = 0;
+  uint32_t ngroups = 0, in_group = 0;
   ViewDesc* h_views = (ViewDesc*)(host + pl.views_off);
   float* h_obj = (float*)(host + pl.objects_off);
   uint32_t item = 0, tile = 0, block = 0;
@@ -740,12 +749,14 @@ void stage_batch(gs3d_pipeline* p, const gs3d_view* views, const Plan& pl, uint3
     p->item_bases[i] = item;
     p->tile_bases[i] = tile;
     const uint32_t b = (d.active_count + kBlock - 1) / kBlock;
-    if (i == 0 || !same_scene(views[i - 1], v)) {
+    if (i == 0 || !same_scene(views[i - 1], v) || in_group == group_views(p, b, n)) {
       h_gblock[ngroups] = block;
       h_gview[ngroups] = i;
       ++ngroups;
       block += b;
+      in_group = 0;
     }
+    ++in_group;
     item += b * kBlock;
     tile += w.tiles_x * w.tiles_y;
     obj += v.camera->object_count;

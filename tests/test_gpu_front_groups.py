@@ -55,3 +55,40 @@ def test_many_views_of_one_scene(views, n, degree):
     for i in (0, views // 2, views - 1):
         o = oracle.render(scene, frames[i], 0)
         assert np.array_equal(front[8 + i], o["rgba"].view(np.uint32))
+
+
+@pytest.mark.parametrize("precision,axis", [("exact", 0), ("half2", 0), ("half2", 1)])
+def test_groups_of_a_large_scene_beside_spread_views_of_a_small_one(precision, axis):
+    # Ten views: five and two of a scene that fills the SMs by itself (a group
+    # each), between them three of a small one (each its own group). Every
+    # view's image is that of its own render, in the batch and in a graph.
+    import torch
+    P = pkg()
+    a, b = (sc.uniform_cloud(n, seed=s, degree=d, log_scale=(-3.0, 0.5)) for n, s, d in ((160001, 42, 1), (3001, 43, 3)))
+    da, db = dev.DeviceScene(a), dev.DeviceScene(b)
+    frames = [sc.make_frame(sc.look_at((11.0 * np.sin(i), 1.0, 11.0 * np.cos(i)), (0, 0, 0)), 128 - 8 * (i % 2), 72,
+                            55.0, 0.1, 100.0, boundary_axis=axis) for i in range(10)]
+    owner = [da] * 5 + [db] * 3 + [da] * 2
+    color = [torch.zeros((f["height"], f["width"], 4), device="cuda") for f in frames]
+    views = [(d.data(), P.make_camera(f), f["width"], f["height"], c.data_ptr(), 0, "rgba32f")
+             for d, f, c in zip(owner, frames, color)]
+    pipe = P.TiledGaussianPipeline(da.data(), pipeline_options(frames[0], precision, 1 << 22))
+
+    def take(call):
+        for c in color:
+            c.zero_()
+        torch.cuda.synchronize()
+        call()
+        assert not pipe.read_stats()["overflow"]
+        return [c.cpu().numpy().view(np.uint32).copy() for c in color]
+
+    images = [take(lambda: pipe.render_batch(views))]
+    stream = torch.cuda.Stream()
+    pipe.capture_graph(views, stream.cuda_stream)
+    images += [take(lambda: pipe.launch_graph([v[1] for v in views], stream=stream.cuda_stream)) for _ in range(2)]
+    for i, v in enumerate(views):
+        alone = take(lambda: pipe.render_batch([v]))[i]
+        assert alone.any()
+        for got in images:
+            assert np.array_equal(got[i], alone), i
+    pipe.dispose()
