@@ -298,13 +298,14 @@ class TiledGaussianPipeline:
         return out
 
     def set_wait_limit(self, polls: int) -> None:
-        """Polls a look-back wait may spend on one status word before the
-        frame reports a device timeout (0: the default, about one second)."""
+        """Polls a wait of the pass's blocks for one another may take before the
+        frame reports a device timeout (0: the default, one to a few seconds;
+        below 65,536 small frames take the separate kernels)."""
         _raise(self._lib, self._lib.gs3d_pipeline_set_wait_limit(self._p, int(polls)), self._p)
 
     def debug_withhold_chunk(self) -> None:
         """Test hook: the next render's compaction never scans its first
-        chunk, so the next chunk's look-back wait runs out."""
+        chunk, so the wait for its sum runs out."""
         _raise(self._lib, self._lib.gs3d_pipeline_debug_withhold_chunk(self._p), self._p)
 
     def debug_refuse_front(self) -> None:

@@ -171,7 +171,7 @@ __device__ __forceinline__ void emit_group(EmitShared& sm, bool live, uint32_t g
   uint32_t nbox = 0, rows = 0;
   if (live) {
     const ViewDesc& v = bv.views[find_view(bv.item_base, bv.nviews, g)];
-    // Emission record: (cx, cy, conic a, b), (conic c, threshold, rx + 512 ry, 0).
+    // Emission record: (cx, cy, conic a, b), (conic c, threshold, rx + 512 ry, tile walk).
     const float4 m = make_float4(e0.x, e0.y, 0.0f, 0.0f), c = make_float4(e0.z, e0.w, e1.x, 0.0f);
     const uint32_t packed = (uint32_t)e1.z;
     const float rx = (float)(packed % 512u), ry = (float)(packed / 512u);

@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(kBlock, kFrontBlocksPerSm) k_front(const __gri
     // of earlier stages, all there; this block is missing at their next one,
     // so each of them comes here.)
     if (tid == 0) {
-      atomicOr(&f.ctl->error, 1u);
+      atomicOr(&f.ctl->error, kErrorWait);
       atomicExch(&f.ctl->state[0], 0u);
       atomicExch(&f.ctl->state[3], 1u);
     }

@@ -140,11 +140,16 @@ struct Control {
   uint32_t tickets[2];           // dynamic chunk ids of the chunked scans (Ticket)
   uint32_t visible_state[4];     // visible, visible, radix blocks, 0
   uint32_t state[4];             // count, total, radix blocks, overflow
-  uint32_t error;                // bit 0: chunk-sum wait or grid barrier expired; bit 2: a sort tile copy never landed
+  uint32_t error;                // ErrorBit
   uint32_t pad[3];
   unsigned long long raster_stats[4];  // checked, blended, pixels, alpha-stopped
   uint32_t order_hist[34];       // raster work-list buckets (tile load classes)
   uint32_t order_fill[34];
+};
+
+enum ErrorBit : uint32_t {
+  kErrorWait = 1u,  // a chunk-sum wait or a grid barrier expired
+  kErrorCopy = 4u   // a sort tile's copy never landed
 };
 
 enum Ticket { kTicketCompact = 0, kTicketScan = 1 };
@@ -183,14 +188,14 @@ __device__ __forceinline__ void st_status(unsigned long long* p, uint32_t epoch,
 __device__ __forceinline__ uint32_t sat_add(uint32_t a, uint32_t b) { return a + min(b, 0xffffffffu - a); }
 
 // Wait (bounded) until *p, last read as v, carries this launch's epoch; its
-// value. On expiry the error word gets bit 0 and the value is zero, so the
+// value. On expiry the error word gets kErrorWait and the value is zero, so the
 // kernel always finishes and the host sees the error.
 __device__ __forceinline__ uint32_t wait_status(const unsigned long long* p, unsigned long long v, uint32_t epoch,
                                                 uint32_t limit, uint32_t* err) {
   uint32_t polls = 0, backoff = 8;
   while ((uint32_t)(v >> 32) != epoch) {
     if (++polls >= limit) {
-      atomicOr(err, 1u);
+      atomicOr(err, kErrorWait);
       return 0;
     }
     __nanosleep(backoff);
@@ -278,8 +283,7 @@ constexpr uint32_t kSumChunks = 16;
 constexpr uint32_t kSumWords = 512;
 __host__ __device__ constexpr uint32_t sum_rows(uint32_t chunks) { return (chunks + kSumChunks - 1u) / kSumChunks; }
 uint32_t chunk_pass_chunks(uint32_t n_max, int sms);
-// err: the control block's error word (bit 2: a tile copy of the scatter
-// never landed).
+// err: the control block's error word (kErrorCopy).
 void launch_chunk_pass(int bits, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
                        uint32_t* vals_out, const uint32_t* n_ptr, uint32_t low, int shift, uint32_t chunks,
                        uint32_t* counts, uint32_t* sums, uint32_t* spare, uint32_t* err, cudaStream_t st);

@@ -287,7 +287,7 @@ gs3d_status ensure_status(gs3d_pipeline* p) {
   if (e == cudaSuccess) e = cudaMemset(fresh, 0, need * sizeof(unsigned long long));
   if (e != cudaSuccess) {
     dfree(fresh);
-    return cuda_fail(p, e, "allocating look-back status");
+    return cuda_fail(p, e, "allocating the scans' status words");
   }
   dfree(p->status);
   p->status = fresh;
@@ -938,7 +938,7 @@ void record_batch(gs3d_pipeline* p, const Plan& pl, unsigned char* dev, cudaStre
   launch_scan_counts(p->dv[cur], p->counts, p->ordered, p->ioff, ctl, p->status, epoch(), cap32, bv.frame_params,
                      p->output_state, scan_grid, st);
   ++launches;
-  // Emission + tile-sort histograms.
+  // Emission.
   mark(p, GS3D_STAGE_EMIT, st);
   launch_emit(p->dv[cur], N, p->erec, p->ordered, p->ioff, bv, o, ctl, cap32, p->tk[0], p->tv[0], st);
   launches += N ? 1 : 0;
@@ -1324,7 +1324,8 @@ gs3d_status fill_stats(gs3d_pipeline* p, const unsigned char* counters, const Ba
   out->raster_pixels = c.raster_stats[2];
   out->raster_alpha_stopped = c.raster_stats[3];
   for (int i = 0; i < 4; ++i) out->output_state[i] = output_state[i];
-  if (c.error) return fail(p, GS3D_ERROR_DEVICE_TIMEOUT, "a device-side look-back wait expired");
+  if (c.error & kErrorWait) return fail(p, GS3D_ERROR_DEVICE_TIMEOUT, "a device-side wait for other blocks expired");
+  if (c.error) return fail(p, GS3D_ERROR_DEVICE_TIMEOUT, "a device-side copy of a sort tile never landed");
   return GS3D_OK;
 }
 

@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kScatterThreads, kChunkBlocksPerSm)
     if (!ok) {
       // A copy never landed: flag the frame and leave, after the copy of the
       // next keys (if one was issued) had its own bounded wait.
-      if (tid == 0) atomicOr(err, 4u);
+      if (tid == 0) atomicOr(err, kErrorCopy);
       if (t + 1u < t1) bar_wait(smem_addr(&s_bar[k ^ 1u]), (phases >> (k ^ 1u)) & 1u);
       return;
     }

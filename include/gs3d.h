@@ -43,7 +43,8 @@ typedef enum gs3d_status {
   GS3D_ERROR_OUT_OF_MEMORY = 4,
   /* Any other CUDA runtime failure. */
   GS3D_ERROR_CUDA = 5,
-  /* A bounded device-side wait (scan/sort look-back) gave up; the frame is invalid. */
+  /* A bounded device-side wait (for other blocks, or for a sort tile's copy)
+   * gave up; the frame is invalid. */
   GS3D_ERROR_DEVICE_TIMEOUT = 6,
   /* The build does not support the requested option. */
   GS3D_ERROR_UNSUPPORTED = 7,

@@ -101,6 +101,7 @@ def test_front_barrier_expires_and_pipeline_recovers(n):
         run.pipe.read_stats()
     assert time.time() - t0 < 30.0  # the kernel returned on its own
     assert err.value.status == P.abi.GS3D_ERROR_DEVICE_TIMEOUT
+    assert "wait for other blocks expired" in str(err.value)
     assert run.pipe.last_launch_count() == 2
     assert (color == 0.25).all() and (depth == 0.5).all()
     # The hook applies to one render only; the next frames are complete and exact.
