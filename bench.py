@@ -150,6 +150,16 @@ class Clocks:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
+def depth_sort_passes(frames: list) -> int:
+    """Radix passes of a direct launch's float32 depth sort over these views:
+    9-bit digits of key - near where the depth planes' range takes three passes
+    or fewer, else four of 8 bits (pipeline.cu: depth_digits)."""
+    import numpy as np
+    low, high = (int(f(np.float32(v[k]) for v in frames).view(np.uint32)) for f, k in ((min, "near"), (max, "far")))
+    passes = (max(1, (high - low).bit_length()) + 8) // 9
+    return min(passes, 4)
+
+
 def stage_bytes(stage: str, n: int, v: int, inter: int, tiles: int, pixels: int, coeffs: int, depth_passes: int,
                 tile_passes: int, color_bytes: int, depth_out: bool, groups: int = 1, precision: str = "half2",
                 views: int = 1) -> int:
@@ -692,8 +702,8 @@ def main() -> None:
     ltile_bits = max(1, int(np.ceil(np.log2(tiles * min(vpl, ncam) + 1))))
     btile_passes = min(4, (ltile_bits + int(tuning["tile_digit_bits"]) - 1) // int(tuning["tile_digit_bits"]))
     for name, ms in stage_ms.items():
-        b = stage_bytes(name, bn, bv_, bi, bt, W * H * ncam, 16, 4, btile_passes, 8, False, groups=nlaunch,
-                        precision=args.precision, views=ncam)
+        b = stage_bytes(name, bn, bv_, bi, bt, W * H * ncam, 16, depth_sort_passes(frames), btile_passes, 8, False,
+                        groups=nlaunch, precision=args.precision, views=ncam)
         gbs = b / (ms * 1e-3) / 1e9 if ms > 0 else 0.0
         stages[name] = {"ms": ms, "bytes": b, "GB/s": gbs, "frac": gbs / hbm}
     dom = max(stages, key=lambda k: stages[k]["ms"])
