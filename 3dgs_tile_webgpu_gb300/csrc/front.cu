@@ -6,8 +6,8 @@
 // Why: a launch of up to a few hundred thousand ordinals keeps each of those
 // kernels busy for 2-5 us, below the cost of a launch (about 4 us of host time
 // and 2-5 us of ramp-up and drain on the GPU each); a grid barrier costs
-// 1-2 us. Whole frames at 1280x720, separate kernels / front: 2000 splats 120 /
-// 62 us, 60k 138 / 87, 200k 189 / 153; the two meet near 400k ordinals.
+// 1-2 us. Whole frames at 1280x720, separate kernels / front: 2000 splats 118 /
+// 61 us, 60k 137 / 86, 200k 188 / 151 (pipeline.cu: kFrontMaxItems).
 //
 // Every buffer ends up with the same contents as after the separate kernels.
 // What differs is how the stages split the work:

@@ -112,7 +112,7 @@ constexpr uint32_t kPackBlock = 256;  // splats, and threads, of a block
 // of a thread are in flight (2 and 8: 56 and 70 us against 60 at degree 2, 76
 // and 81 against 76 at degree 3).
 // 1M splats at degree 3: 1810 us with a thread per splat and the double
-// log1p, 95 us with the words spread, 76 us (4.3 TB/s) so; 4M 322 and 261 us.
+// log1p, 90 us with the words spread, 72 us (4.6 TB/s) so; 4M 322 and 261 us.
 template <uint32_t C>
 __global__ void __launch_bounds__(kPackBlock) k_pack(gs3d_splat_source src, uint32_t first,
                                                      float4* __restrict__ means, uint2* __restrict__ shape,

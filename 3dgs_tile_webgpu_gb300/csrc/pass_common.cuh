@@ -163,7 +163,7 @@ enum Ticket { kTicketCompact = 0, kTicketScan = 1 };
 // so a replayed CUDA graph never reuses an epoch.
 constexpr uint32_t kEpochsPerFrame = 16;
 
-constexpr uint32_t kSpinLimit = 1u << 22;  // default polls before a wait is declared expired (about 1 s)
+constexpr uint32_t kSpinLimit = 1u << 22;  // default polls before a wait is declared expired (one to a few seconds)
 
 // The epoch of chunked-scan launch `add` of the current frame, and how many
 // polls a wait of that launch may spend on one status word.

@@ -774,12 +774,17 @@ void stage_batch(gs3d_pipeline* p, const gs3d_view* views, const Plan& pl, uint3
 }
 
 // Launches of up to this many ordinals take the fused front (front.cu): its
-// three blocks per SM project and sort slower than the separate kernels, but
-// it saves their launches. Frames of n ordinals at 1280x720 / 1920x1080, us,
-// front against separate kernels: 2k 62 / 120 and 72 / 127, 60k 87 / 138 and
-// 100 / 149, 200k 153 / 189 and 172 / 198, 330k 197 / 229 and 210 / 241, 400k
-// 224 / 254 and 288 / 261 (with a clustered scene 277 / 289 and 258 / 258),
-// 520k 310 / 288 and 348 / 291, 1M 533 / 394 and 554 / 401.
+// three blocks per SM project, emit and sort slower than the separate kernels,
+// but it saves their launches. Front / separate kernels, us, n uniform splats
+// with 2-2.4 records each at 1280x720 and 1920x1080, 4 each at 3840x2160:
+//   2k    61 / 118   67 / 125  124 / 174     393k  221 / 248  254 / 258  382 / 370
+//   60k   86 / 137   99 / 149  175 / 209     520k  276 / 295  292 / 297  444 / 442
+//   200k 151 / 188  166 / 202  260 / 283     1M    410 / 391  425 / 407  639 / 588
+//   330k 196 / 234  209 / 245  340 / 340
+// What the host cannot see, the records per splat, moves the crossover down:
+// with 4-14 each, 200k 174 / 204, 226 / 234 and 406 / 400, 393k 249 / 247,
+// 300 / 291 and 543 / 500; with 24 and more the separate kernels are up to 1.4
+// times as quick. Before the front all of these took longer than either.
 constexpr uint32_t kFrontMaxItems = 3u << 17;
 
 // A barrier of the front waits for its slowest block's whole stage, some

@@ -63,7 +63,8 @@ std::atomic<bool> g_refuse_finish{false};
 // counter wraps, with every status word cleared, so that no word left by an
 // earlier call can carry a later one's epoch). Bound by its launch; a kernel
 // that advanced the epoch, a memset and two copies took four: 1000 keys 23.2
-// -> 13.0 us, 100k 32.5 -> 20.1, 5M 47.8 -> 33.4 (with the chunks' sums).
+// -> 13.0 us, 100k 32.5 -> 20.1, 5M 40.6 -> 30.3 (with the chunks' sums; 27 with
+// overlapped launches).
 __global__ void __launch_bounds__(256) k_static_finish(Control* ctl, unsigned long long* status, uint32_t* epoch,
                                                        unsigned char* result) {
   after_previous();
