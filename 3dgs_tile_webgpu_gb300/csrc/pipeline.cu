@@ -789,7 +789,7 @@ constexpr uint32_t kFrontMaxItems = 3u << 17;
 
 // A barrier of the front waits for its slowest block's whole stage, some
 // microseconds to a few milliseconds, a chunk-sum wait of the separate kernels
-// for a sum that is about to come. Set wait limits below this (about 60 ms of
+// for a sum that is about to come. Set wait limits below this (about 33 ms of
 // the barriers' polls) keep the kernels whose waits they were made for; a
 // working frame could run out of them in the front.
 constexpr uint32_t kFrontMinPolls = 1u << 16;

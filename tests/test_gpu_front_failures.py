@@ -66,7 +66,7 @@ def test_refused_front_in_a_captured_graph():
     run.close()
 
 
-LIMIT = 1 << 16  # polls: the shortest limit that the front's barriers take, some 60 ms
+LIMIT = 1 << 16  # polls: the shortest limit that the front's barriers take, some 33 ms
 
 
 def test_front_takes_set_limits_that_its_barriers_can_keep():
